@@ -412,7 +412,8 @@ int buildPrograms(QuregState &s, int W, std::vector<TileProgram> &out, PlanStats
         p.denseOff = (uint32_t) s.denseHost.size();
         for (int i = 0; i < g.numMultiTargets; i++) p.denseTargets[i] = (uint8_t) g.multiTargets[i];
         const auto &m = s.pool.mats[(size_t) g.multiIndex];
-        s.denseHost.insert(s.denseHost.end(), m.begin(), m.end());
+        s.denseHost.resize(s.denseHost.size() + m.size());
+        packDenseMatrix(g.numMultiTargets, m.data(), s.denseHost.data() + p.denseOff);
         if (s.single && tcBlockSupported(s.numBits, g.numMultiTargets)) {
             // the pipelined tensor-core operand ([Whi | Wlo], FP16) in the doubles buffer
             const size_t nf = tcBlockMatrixFloats(g.numMultiTargets);
@@ -465,7 +466,7 @@ void consumePending(QuregState &s) {
 namespace dgq_api {
 
 // Dense 6-target unitaries on complex64 registers run on the tensor cores
-// (dgq_setTensorCores(0): the SIMT dense kernel instead).
+// (dgq_setTensorCores(0): the FP64 dense kernel instead).
 
 // 0: compile specialised kernels when a plan needs them; 1: specialise only
 // plans whose kernels are compiled already, interpret the others while

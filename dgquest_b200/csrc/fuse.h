@@ -1,6 +1,6 @@
 // fuse.h -- the dense-block form: recorded gates fused into dense unitaries
 // on K qubits, each applied as one dense sweep (a complex GEMM over the
-// state: on the tensor cores for complex64 registers and K = 6, the SIMT
+// state: on the tensor cores for complex64 registers and K = 6, the FP64
 // dense kernel otherwise).
 //
 // Blocks are chosen with dgQuEST's greedy rule (DAG.cpp:219-259: take every

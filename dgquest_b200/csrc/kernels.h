@@ -85,7 +85,9 @@ struct DenseArgs {
 };
 // Fills the tile map for K targets (targets[i] = address bit of matrix bit i).
 bool denseArgs(int numBits, int K, const uint8_t *targets, DenseArgs &a);
-// U: 2^K x 2^K row-major, (re, im) interleaved FP64, in device memory.
+// U: the matrix in fragment order (packDenseMatrix; 2 x 4^K doubles), in
+// device memory, 16-byte aligned.
+void packDenseMatrix(int K, const double *U, double *out);
 cudaError_t launchDense(void *st, bool single, int K, const DenseArgs &a, const double *U, cudaStream_t s);
 
 // Tensor-core form for complex64 and 6 targets (tc_dense.cu): the matrix is

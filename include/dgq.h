@@ -142,8 +142,8 @@ int dgq_getShardStats(Qureg qureg, int *shardBits, int64_t *passes, int64_t *exc
  * on that many qubits (dgQuEST's greedy block rule, DAG.cpp:219-259, with
  * every qubit a gate touches counted), composed in FP64 on the host and
  * applied one per sweep as a complex GEMM over the state: on the tensor
- * cores (tcgen05, 3xTF32) for complex64 registers and 6 qubits, the SIMT
- * dense kernel otherwise. 0 runs gates in register-phase sweeps. -1 (the
+ * cores (tcgen05) for complex64 registers and 5 or 6 qubits, the FP64 matrix
+ * instruction otherwise. 0 runs gates in register-phase sweeps. -1 (the
  * default) lets the cost model choose per plan between the register-phase
  * tiles (and their width) and dense blocks of 5, 6 or 7 qubits; the plan
  * statistics report the choice (formK) and every prediction. Registers of
@@ -249,7 +249,7 @@ int dgq_setSpecialisationMinBits(int minBits);
 int dgq_setSpecialisationPolicy(int policy);
 /* multiQubitUnitary with 6 targets on a complex64 register of >= 12 qubits
  * runs on the tensor cores (tcgen05, 3xTF32 split, FP32 accumulation) when
- * enabled (default 1); 0 selects the SIMT dense kernel. Returns the previous
+ * enabled (default 1); 0 selects the FP64 dense kernel. Returns the previous
  * setting. */
 int dgq_setTensorCores(int enable);
 /* Nonzero when a tensor-core sweep stopped waiting for its MMAs (bounded
