@@ -99,20 +99,60 @@ CostModel costModel() {
     return g_cost;
 }
 
+// A unitary with more targets than a register phase holds runs as a dense
+// sweep of its own, whatever the tile width.
+bool isWide(const Gate &g) { return g.type == dgq::OP_MULTI_UNITARY && g.numMultiTargets > dgq::kRegBits; }
+
+// The tile sweeps of the gates: those between two wide unitaries are planned
+// by themselves, as buildPrograms does. (Planned as one list, a wide unitary
+// stopped the count of a width it exceeds and failed the encoding of the
+// others, so the tile form lost to dense blocks: 26 qubits, one layer and
+// four 6-qubit unitaries, 7 extra dense sweeps of 0.81 ms for 3 tile sweeps
+// of 0.34 ms.)
 double predictPlanSeconds(const std::vector<Gate> &gates, int numBits, int W, const dgq::MatrixPool &pool,
                           int lookahead) {
     const CostModel cm = costModel();
-    std::vector<dgq::BlockPlan> blocks = dgq::planBlocks(gates, numBits, W, nullptr, dgq::kCoalescedBits, lookahead);
     const double amps = std::ldexp(1.0, numBits);
     std::vector<dgq::TileProgram> progs;
     dgq::PlanStats st;
     dgq::SweepHeader h;
     std::string err;
-    for (const auto &b : blocks) {
-        progs.clear();
-        if (!dgq::encodeBlock(b, numBits, numBits, W, pool, h, progs, &st, &err)) return 1e30;
+    auto count = [&](const std::vector<Gate> &seg) {
+        for (const auto &b : dgq::planBlocks(seg, numBits, W, nullptr, dgq::kCoalescedBits, lookahead)) {
+            progs.clear();
+            if (!dgq::encodeBlock(b, numBits, numBits, W, pool, h, progs, &st, &err)) return false;
+        }
+        return true;
+    };
+    if (std::none_of(gates.begin(), gates.end(), isWide)) {
+        if (!count(gates)) return 1e30;
+    } else {
+        std::vector<Gate> seg;
+        for (size_t i = 0; i <= gates.size(); i++) {
+            if (i < gates.size() && !isWide(gates[i])) {
+                seg.push_back(gates[i]);
+                continue;
+            }
+            if (!seg.empty() && !count(seg)) return 1e30;
+            seg.clear();
+        }
     }
     return st.sweeps * (amps * cm.sweepSecondsPerAmp + cm.launchSeconds) + st.phases * amps * cm.phaseSecondsPerAmp;
+}
+
+// One dense sweep of K targets on a register like s.
+double denseSweepSeconds(const QuregState &s, int K, const CostModel &cm) {
+    const bool tensor = s.single && g_tensorCores.load() && cm.denseMs[DV_C64_TC][K - 5] > 0.0;
+    const double ms = cm.denseMs[!s.single ? DV_F64 : tensor ? DV_C64_TC : DV_C64][K - 5];
+    return ms * 1e-3 * std::ldexp(1.0, s.numBits) / 1073741824.0 + cm.launchSeconds;
+}
+
+// The dense sweeps of the wide unitaries with more than K targets.
+double wideSeconds(const QuregState &s, const std::vector<Gate> &gates, int K, const CostModel &cm) {
+    double t = 0.0;
+    for (const Gate &g : gates)
+        if (isWide(g) && g.numMultiTargets > K) t += denseSweepSeconds(s, g.numMultiTargets, cm);
+    return t;
 }
 
 int chooseTileBits(QuregState &s) {
@@ -166,16 +206,13 @@ int chooseTileBits(QuregState &s) {
 }
 
 // Predicted time of the dense-block form with K-qubit blocks: the blocks'
-// dense sweeps plus the tile sweeps of the gates that touch more than K
-// qubits and pass through. *blocksOut: the number of blocks.
+// dense sweeps plus the sweeps of the gates that touch more than K qubits
+// and pass through. *blocksOut: the number of blocks.
 // bound > 0: stop counting blocks once they cost more than bound seconds
 // (*stopped is set and the result is the cost of the blocks counted).
 double predictDenseSeconds(const QuregState &s, int K, int *blocksOut, double bound, bool *stopped) {
     const CostModel cm = costModel();
-    const int var = !s.single ? DV_F64 : (K == 6 && g_tensorCores.load() ? DV_C64_TC : DV_C64);
-    const double rate = cm.denseMs[var][K - 5] > 0.0 ? cm.denseMs[var][K - 5] : cm.denseMs[DV_C64][K - 5];
-    const double amps = std::ldexp(1.0, s.numBits);
-    const double perBlock = rate * 1e-3 * amps / 1073741824.0 + cm.launchSeconds;
+    const double perBlock = denseSweepSeconds(s, K, cm);
     const int maxBlocks = bound > 0.0 ? (int) std::min(1e6, std::floor(bound / perBlock)) + 1 : 0;
     dgq::MatrixPool pool = s.pool;
     int blocks = 0;
@@ -187,12 +224,12 @@ double predictDenseSeconds(const QuregState &s, int K, int *blocksOut, double bo
     if (cut) return t;
     std::vector<Gate> rest;
     for (const Gate &g : fused)
-        if (!(g.type == dgq::OP_MULTI_UNITARY && g.numMultiTargets > dgq::kRegBits)) rest.push_back(g);
+        if (!isWide(g)) rest.push_back(g);
     if (!rest.empty()) {
         const double tt = predictPlanSeconds(rest, s.numBits, std::min(12, s.numBits), pool, -1);
         t += s.single ? tt * cm.c64TileFactor : tt;
     }
-    return t;
+    return t + wideSeconds(s, fused, K, cm);
 }
 
 // The predictor's choice of form for the pending gates (dgq_setDenseFusion
@@ -271,6 +308,7 @@ int chooseFormUncached(QuregState &s, const CostModel &cm) {
     s.formLookahead = s.planLookahead;
     double tile = s.predictedTileSeconds;
     if (s.single) tile *= cm.c64TileFactor;
+    tile += wideSeconds(s, s.pending, dgq::kRegBits, cm);
     s.stats.predictedTileMs = tile * 1e3;
     double dense[3] = {0.0, 0.0, 0.0};
     int blocks[3] = {0, 0, 0};

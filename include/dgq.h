@@ -88,8 +88,8 @@ int dgq_setCostModel(double sweepMsPer2p30, double phaseMsPer2p30);
 int dgq_loadCostModel(const char *path);
 int dgq_getCostModel(double *sweepMsPer2p30, double *phaseMsPer2p30);
 /* Rates of the dense-block forms in the form choice: ms per dense block per
- * 2^30 amplitudes for variant 0 (complex128, SIMT), 1 (complex64, SIMT) or
- * 2 (complex64, tensor cores; K = 6), K = 5..7. A cost file may carry them
+ * 2^30 amplitudes for variant 0 (complex128), 1 (complex64 without tensor cores) or
+ * 2 (complex64, tensor cores; K = 5, 6), K = 5..7. A cost file may carry them
  * as "dense_ms_per_2p30_<f64|c64|c64tc>_k<K> <ms>", and the complex64 tile
  * factor as "c64_tile_factor <x>". Set returns 0 or -1; get returns the
  * rate, or -1 on a bad argument. */

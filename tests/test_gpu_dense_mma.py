@@ -46,3 +46,34 @@ def test_dense_sweep_edges(quest, env, n, targs, single):
     if single:
         bound += 4 * 2.0 ** -24 * np.abs(want).max()
     assert np.abs(got - want).max() <= bound
+
+
+@pytest.mark.parametrize("single", [False, True])
+def test_wide_unitaries_keep_the_tile_form(quest, env, single):
+    """The gates between wide unitaries are priced as tile sweeps, so one
+    layer of rotations is not fused into extra dense sweeps; the chosen plan
+    equals the forced tile form."""
+    Q, n = quest, 22
+    gen = np.random.default_rng(22)
+    first = C.random_layers(n, 1, 5)
+    wide = [(gen.choice(n, k, replace=False).tolist(), C.random_unitary(gen, 1 << k)) for k in (6, 5, 7, 6)]
+
+    def run(form):
+        q = Q.dgq_createQuregF32(n, env) if single else Q.createQureg(n, env)
+        Q.dgq_setDenseFusion(q, form)
+        C.replay(q, first)
+        for targs, u in wide:
+            m = Q.matrixN(u)
+            Q.multiQubitUnitary(q, Q.int_array(targs), len(targs), m)
+            Q.destroyComplexMatrixN(m)
+        amps = Q.state_vector(q)
+        st = Q.plan_stats(q)
+        Q.destroyQureg(q, env)
+        return amps, st
+
+    amps, st = run(-1)
+    assert st.formAuto == 1 and st.formK == 0 and st.denseBlocks == 0
+    assert 0.0 < st.predictedTileMs < 1e3
+    want, _ = run(0)
+    # the two plans may differ in their tile width: rounding of the first layer only
+    assert np.linalg.norm(amps - want) <= (1e-5 if single else 1e-13)
