@@ -92,7 +92,7 @@ struct CostModel {
     double sweepSecondsPerAmp = 2.6e-3 / 1073741824.0;
     double phaseSecondsPerAmp = 1.8e-3 / 1073741824.0;
     double launchSeconds = 3e-6;
-    double denseMs[3][3] = {{12.9, 19.6, 35.1}, {9.6, 17.5, 33.0}, {5.24, 5.5, 0.0}};  // [variant][K - 5]
+    double denseMs[3][3] = {{12.9, 19.6, 35.1}, {11.4, 17.9, 33.0}, {5.24, 5.5, 0.0}};  // [variant][K - 5]
     double c64TileFactor = 0.55;
     double denseMargin = 0.8;
 };

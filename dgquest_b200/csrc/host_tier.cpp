@@ -566,9 +566,9 @@ bool hostTierProbs(QuregState &s, std::vector<double> &p0, double &total, const 
         a.freePos[nf++] = (uint8_t) b;
     }
     a.nFree = nf;
-    a.kappa = std::min(4, std::max(0, nf - 12));
     a.rValue = rValue & localMask;
-    const size_t need = (size_t) probNumCtas(a) * 17;
+    probShape(a, s.single);
+    const size_t need = (size_t) probNumCtas(a) * kProbSlots;
     if (s.sharded && need > s.shardPartialCap) {
         for (int k = 0; k < (1 << s.shardBits); k++) {
             DeviceScope on(s.shardDev[k]);

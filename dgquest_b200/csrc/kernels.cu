@@ -174,101 +174,133 @@ cudaError_t launchTile(void *st, bool single, int tileBits, const TileProgram &p
 // ------------------------------------------------------- probabilities
 // Sub-index s enumerates the amplitudes allowed by the lazy collapse
 // (address bits outside `restrict` mask): address = rValue | deposit(s).
-// s bits 0..7 = thread, 8..11 = register j, 12..12+kappa-1 = unit within
-// the CTA, the rest = blockIdx. Each CTA writes 17 partial sums:
-// [0..7] zero-sums of the thread bits, [8..11] of the j bits,
-// [12..15] of the unit bits, [16] the CTA total.
-template <class V>
-__global__ void __launch_bounds__(256) probKernel(const V *__restrict__ st, const __grid_constant__ ProbArgs args, double *partial) {
+// With VB = 1 (complex64, address bit 0 free) s bit 0 is inside a 16-byte
+// load. Above it 8 bits = thread, 4 = register j, kappa = unit within the
+// CTA, the rest = blockIdx. Each CTA writes kProbSlots partial sums: the
+// zero-sum of sub-index bit i at slot i (inside the CTA), its total last.
+//
+// Bound: HBM (one read of the state). Loads are 16 bytes a lane in either
+// precision, 16 of them in flight; the 16 values are added as a tree whose
+// nodes give the four j sums (26 adds for 16 values instead of 48), and
+// lane-bit sums come out of the warp's butterfly (15 shuffles instead of
+// 45). kappa keeps at least 2048 CTAs where the state has as many units: at
+// 2^21 amplitudes 512 CTAs instead of the 32 that 16 units a CTA left.
+// Measured (us, before -> now): complex128 2^17 61 -> 4.4, 2^21 73 -> 8.9,
+// 2^25 141 -> 106, 2^30 2777 -> 2564 (6.7 TB/s); complex64 2^23 88 -> 15,
+// 2^29 1204 -> 701 (6.1 TB/s).
+template <class V, int VB>
+__global__ void __launch_bounds__(256, 3) probKernel(const V *__restrict__ st, const __grid_constant__ ProbArgs args, double *partial) {
     const uint32_t tid = threadIdx.x;
     const uint32_t cta = blockIdx.x;
     const int nFree = args.nFree;
     const int kappa = args.kappa;
     auto bitOf = [&](int i) -> uint64_t { return i < nFree ? (1ULL << args.freePos[i]) : 0ULL; };
-    uint64_t dTid = 0;
+    uint64_t base = args.rValue;
 #pragma unroll
     for (int i = 0; i < 8; i++)
-        if ((tid >> i) & 1u) dTid |= bitOf(i);
-    uint64_t dCta = 0;
-    for (int i = 0; 12 + kappa + i < nFree; i++)
-        if ((cta >> i) & 1u) dCta |= bitOf(12 + kappa + i);
-    const uint64_t j0 = bitOf(8), j1 = bitOf(9), j2 = bitOf(10), j3 = bitOf(11);
-    const uint64_t limit = nFree >= 63 ? ~0ULL : (1ULL << nFree);
+        if ((tid >> i) & 1u) base |= bitOf(VB + i);
+    for (int i = 0; VB + 12 + kappa + i < nFree; i++)
+        if ((cta >> i) & 1u) base |= bitOf(VB + 12 + kappa + i);
+    const uint64_t jb[4] = {bitOf(VB + 8), bitOf(VB + 9), bitOf(VB + 10), bitOf(VB + 11)};
+    // registers narrower than one unit: only sub-indices below 2^nFree exist
+    const bool full = nFree >= VB + 12;
+    const uint32_t limit = full ? 0u : 1u << (nFree > VB ? nFree - VB : 0);
 
-    double tot = 0.0, zj0 = 0.0, zj1 = 0.0, zj2 = 0.0, zj3 = 0.0;
-    double zu[4] = {0.0, 0.0, 0.0, 0.0};
+    double tot = 0.0, zb = 0.0;       // zb: sub-index bit 0 = 0 (VB = 1)
+    double zj[4] = {0.0, 0.0, 0.0, 0.0};
+    double zu[kProbMaxKappa] = {};
     const int units = 1 << kappa;
     for (int u = 0; u < units; u++) {
-        uint64_t dU = 0;
+        uint64_t g0 = base;
         for (int b = 0; b < kappa; b++)
-            if ((u >> b) & 1) dU |= bitOf(12 + b);
-        const uint64_t gbase = args.rValue | dCta | dU | dTid;
-        const uint64_t sbase = ((((uint64_t) cta << kappa) | (uint64_t) u) << 12) | tid;
-        double ut = 0.0;
+            if ((u >> b) & 1) g0 |= bitOf(VB + 12 + b);
+        double p[16], lo = 0.0;
 #pragma unroll
         for (int j = 0; j < 16; j++) {
-            const uint64_t s = sbase | ((uint64_t) j << 8);
-            const uint64_t g = gbase | ((j & 1) ? j0 : 0ULL) | ((j & 2) ? j1 : 0ULL) | ((j & 4) ? j2 : 0ULL) | ((j & 8) ? j3 : 0ULL);
-            double p = 0.0;
-            if (s < limit) {
-                const V v = st[g];
-                const double re = (double) v.x, im = (double) v.y;
-                p = re * re + im * im;
+            const uint64_t g = g0 | ((j & 1) ? jb[0] : 0ULL) | ((j & 2) ? jb[1] : 0ULL) | ((j & 4) ? jb[2] : 0ULL) |
+                               ((j & 8) ? jb[3] : 0ULL);
+            p[j] = 0.0;
+            if (full || (tid | ((uint32_t) j << 8)) < limit) {
+                if constexpr (VB == 1) {
+                    const float4 v = *reinterpret_cast<const float4 *>(st + g);
+                    const double ar = (double) v.x, ai = (double) v.y, br = (double) v.z, bi = (double) v.w;
+                    const double l = ar * ar + ai * ai;
+                    lo += l;
+                    p[j] = l + (br * br + bi * bi);
+                } else {
+                    const V v = st[g];
+                    const double re = (double) v.x, im = (double) v.y;
+                    p[j] = re * re + im * im;
+                }
             }
-            ut += p;
-            if (!(j & 1)) zj0 += p;
-            if (!(j & 2)) zj1 += p;
-            if (!(j & 4)) zj2 += p;
-            if (!(j & 8)) zj3 += p;
         }
+        zb += lo;
+        double a[8], c[4];
+#pragma unroll
+        for (int i = 0; i < 8; i++) a[i] = p[2 * i] + p[2 * i + 1];
+#pragma unroll
+        for (int i = 0; i < 4; i++) c[i] = a[2 * i] + a[2 * i + 1];
+        zj[0] += ((p[0] + p[2]) + (p[4] + p[6])) + ((p[8] + p[10]) + (p[12] + p[14]));
+        zj[1] += (a[0] + a[2]) + (a[4] + a[6]);
+        zj[2] += c[0] + c[2];
+        zj[3] += c[0] + c[1];
+        const double ut = (c[0] + c[1]) + (c[2] + c[3]);
         tot += ut;
 #pragma unroll
-        for (int b = 0; b < 4; b++)
+        for (int b = 0; b < kProbMaxKappa; b++)
             if (b < kappa && !((u >> b) & 1)) zu[b] += ut;
     }
-    double v[17];
-#pragma unroll
-    for (int i = 0; i < 8; i++) v[i] = ((tid >> i) & 1u) ? 0.0 : tot;
-    v[8] = zj0;
-    v[9] = zj1;
-    v[10] = zj2;
-    v[11] = zj3;
-#pragma unroll
-    for (int b = 0; b < 4; b++) v[12 + b] = zu[b];
-    v[16] = tot;
-    __shared__ double red[8][17];
+    // per warp: [0..5) lane bits, 5 total, 6 bit 0 of a pair, [7..11) j, [11..) units
+    __shared__ double red[8][11 + kProbMaxKappa];
     const int lane = tid & 31, warp = tid >> 5;
+    double z[5], sum = tot;
 #pragma unroll
-    for (int i = 0; i < 17; i++) {
-        double x = v[i];
+    for (int k = 0; k < 5; k++) {
+        const double other = __shfl_xor_sync(0xffffffffu, sum, 1 << k);
+        z[k] = ((lane >> k) & 1) ? other : sum;
+        sum += other;
+#pragma unroll
+        for (int i = 0; i < k; i++) z[i] += __shfl_xor_sync(0xffffffffu, z[i], 1 << k);
+    }
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) red[warp][k] = z[k];
+        red[warp][5] = sum;
+    }
+    auto reduce = [&](double x, int slot) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane == 0) red[warp][i] = x;
-    }
+        if (lane == 0) red[warp][slot] = x;
+    };
+    if constexpr (VB == 1) reduce(zb, 6);
+#pragma unroll
+    for (int k = 0; k < 4; k++) reduce(zj[k], 7 + k);
+#pragma unroll
+    for (int b = 0; b < kProbMaxKappa; b++)
+        if (b < kappa) reduce(zu[b], 11 + b);
     __syncthreads();
-    if (tid < 17) {
+    const int inside = VB + 12 + kappa;
+    if ((int) tid < inside || tid == kProbSlots - 1) {
+        const int i = (int) tid - VB;  // sub-index bit above the load
+        const bool warpBit = tid != kProbSlots - 1 && i >= 5 && i < 8;
+        const int slot = tid == kProbSlots - 1 || warpBit ? 5 : i < 0 ? 6 : i < 5 ? i : i - 1;
         double x = 0.0;
 #pragma unroll
-        for (int w = 0; w < 8; w++) x += red[w][tid];
-        partial[(size_t) cta * 17 + tid] = x;
+        for (int w = 0; w < 8; w++)
+            if (!warpBit || !((w >> (i - 5)) & 1)) x += red[w][slot];
+        partial[(size_t) cta * kProbSlots + tid] = x;
     }
 }
 
 // out[b] for sub-index bit b < nFree, out[nFree] = total.
 __global__ void __launch_bounds__(256) probFinalize(const double *__restrict__ partial, int numCtas, int nFree,
-                                                   int kappa, double *out) {
+                                                   int inside, double *out) {
     const int b = blockIdx.x;  // 0..nFree
     double x = 0.0;
-    const int local = 12 + kappa;
-    for (int c = threadIdx.x; c < numCtas; c += blockDim.x) {
-        if (b == nFree) {
-            x += partial[(size_t) c * 17 + 16];
-        } else if (b < local) {
-            x += partial[(size_t) c * 17 + b];
-        } else if (!((c >> (b - local)) & 1)) {
-            x += partial[(size_t) c * 17 + 16];
-        }
-    }
+    const int slot = b < nFree && b < inside ? b : kProbSlots - 1;
+    const int skip = b < nFree && b >= inside ? 1 << (b - inside) : 0;
+    for (int c = threadIdx.x; c < numCtas; c += blockDim.x)
+        if (!(c & skip)) x += partial[(size_t) c * kProbSlots + slot];
     __shared__ double red[8];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
@@ -281,21 +313,30 @@ __global__ void __launch_bounds__(256) probFinalize(const double *__restrict__ p
     }
 }
 
+void probShape(ProbArgs &args, bool single) {
+    args.pairs = single && args.nFree > 0 && args.freePos[0] == 0 ? 1 : 0;
+    const int unitBits = std::max(0, args.nFree - 12 - args.pairs);
+    args.kappa = std::min(kProbMaxKappa, std::max(0, unitBits - 11));
+}
+
 cudaError_t launchProb(const void *st, bool single, const ProbArgs &args, double *partial, double *out,
                        cudaStream_t s) {
-    const int grid = args.nFree > 12 + args.kappa ? (1 << (args.nFree - 12 - args.kappa)) : 1;
-    if (single)
-        probKernel<float2><<<grid, 256, 0, s>>>((const float2 *) st, args, partial);
+    const int grid = probNumCtas(args);
+    if (single && args.pairs)
+        probKernel<float2, 1><<<grid, 256, 0, s>>>((const float2 *) st, args, partial);
+    else if (single)
+        probKernel<float2, 0><<<grid, 256, 0, s>>>((const float2 *) st, args, partial);
     else
-        probKernel<double2><<<grid, 256, 0, s>>>((const double2 *) st, args, partial);
+        probKernel<double2, 0><<<grid, 256, 0, s>>>((const double2 *) st, args, partial);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    probFinalize<<<args.nFree + 1, 256, 0, s>>>(partial, grid, args.nFree, args.kappa, out);
+    probFinalize<<<args.nFree + 1, 256, 0, s>>>(partial, grid, args.nFree, 12 + args.pairs + args.kappa, out);
     return cudaGetLastError();
 }
 
 int probNumCtas(const ProbArgs &args) {
-    return args.nFree > 12 + args.kappa ? (1 << (args.nFree - 12 - args.kappa)) : 1;
+    const int inside = 12 + args.pairs + args.kappa;
+    return args.nFree > inside ? (1 << (args.nFree - inside)) : 1;
 }
 
 // Page-pair exchange of the host tier: pages a and b differ only in the

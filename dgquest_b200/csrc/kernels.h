@@ -31,9 +31,13 @@ inline cudaError_t ensureSmemOptIn(const void *func, int bytes, std::atomic<uint
 
 namespace dgq {
 
+constexpr int kProbMaxKappa = 6;
+constexpr int kProbSlots = 20;  // partial sums per CTA: at most 1 + 12 + kProbMaxKappa bits, and the total
+
 struct ProbArgs {
     int32_t nFree;     // address bits not fixed by the lazy collapse
-    int32_t kappa;     // log2 of 4096-amplitude units per CTA (0..4)
+    int32_t kappa;     // log2 of the units per CTA (4096 loads each)
+    int32_t pairs;     // 1: a load holds two complex64 amplitudes
     uint64_t rValue;   // fixed bits' values
     uint8_t freePos[kMaxStateBits];  // address bit of sub-index bit i
 };
@@ -130,6 +134,9 @@ int innerNumCtas();
 cudaError_t launchTile(void *st, bool single, int tileBits, const TileProgram &prog, cudaStream_t s);
 cudaError_t launchProb(const void *st, bool single, const ProbArgs &args, double *partial, double *out,
                        cudaStream_t s);
+// Sets kappa and pairs from nFree and freePos; partial then holds
+// kProbSlots * probNumCtas doubles.
+void probShape(ProbArgs &args, bool single);
 int probNumCtas(const ProbArgs &args);
 // Exchanges address bits a[k] <-> b[k] (disjoint pairs) of the whole state, in place.
 cudaError_t launchSwapBits(void *st, bool single, const SwapArgs &args, cudaStream_t s);

@@ -99,10 +99,10 @@ extern "C" int dgq_calcProbOfAllZeroNoAlloc(const void *deviceState, int numBits
     }
     ProbArgs a;
     a.nFree = numBits;
-    a.kappa = numBits > 16 ? 4 : (numBits > 12 ? numBits - 12 : 0);
     a.rValue = 0;
     for (int i = 0; i < kMaxStateBits; i++) a.freePos[i] = (uint8_t) (i < numBits ? i : 0);
-    if (probNumCtas(a) > kStaticProbCtas) {
+    probShape(a, false);
+    if ((size_t) probNumCtas(a) * kProbSlots > sizeof(g_probScratch) / sizeof(double)) {
         raiseExternal(104, __func__, "state larger than the static scratch holds");
         return -1;
     }

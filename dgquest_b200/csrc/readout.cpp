@@ -97,9 +97,9 @@ bool ensureProbs(QuregState &s, const char *func) {
         a.freePos[nf++] = (uint8_t) b;
     }
     a.nFree = nf;
-    a.kappa = std::min(4, std::max(0, nf - 12));
     a.rValue = s.restrictActive ? s.rValue : 0;
-    const size_t need = (size_t) dgq::probNumCtas(a) * 17;
+    dgq::probShape(a, s.single);
+    const size_t need = (size_t) dgq::probNumCtas(a) * dgq::kProbSlots;
     if (need > s.partialCap) {
         freeOn(s.dPartial, s.stream);
         s.dPartial = nullptr;
