@@ -374,7 +374,7 @@ int jitMinBits() {
 namespace dgq {
 
 int buildPrograms(QuregState &s, int W, std::vector<TileProgram> &out, PlanStats &st, std::string &err,
-                  bool paired, const std::function<bool(size_t)> &emit) {
+                  bool paired, const std::function<bool(size_t)> &emit, bool folds) {
     // hands the programs from index `from` on to emit
     auto emitted = [&](size_t from) -> bool {
         if (!emit) return true;
@@ -402,12 +402,13 @@ int buildPrograms(QuregState &s, int W, std::vector<TileProgram> &out, PlanStats
     auto planSegment = [&]() -> int {
         if (seg.empty()) return 0;
         int code = 0;
+        std::vector<Gate> carry;
         const bool complete = planBlocksEach(seg, s.numBits, W, paired ? kCoalescedBits + 1 : kCoalescedBits,
                                              [&](BlockPlan &b) {
                                                  SweepHeader hb = first ? h : SweepHeader();
                                                  const size_t from = out.size();
                                                  if (!encodeBlock(b, s.numBits, s.numQubits, W, s.pool, hb, out, &st,
-                                                                  &err, paired)) {
+                                                                  &err, paired, folds, folds ? &carry : nullptr)) {
                                                      code = E_UNSUPPORTED;
                                                      return false;
                                                  }
@@ -667,7 +668,7 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
         st = dgq::PlanStats();
         err.clear();
         event = 0;
-        int code = dgq::buildPrograms(s, W, s.planned, st, err, paired, emit);
+        int code = dgq::buildPrograms(s, W, s.planned, st, err, paired, emit, !interpret);
         if (code) return code;
         const size_t last = s.planned.size() - 1;
         for (size_t i = launched; i <= last; i++) setRenorm(s, i, last, event);
@@ -692,12 +693,11 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
             }
         if (cachedOnly && !dgq::jitAllReady(sources)) {
             if (policy == 1) dgq::jitCompileInBackground(sources);
-            if (paired || W > dgq::kMaxTileBitsF64) {
-                // the interpreting kernel runs unpaired programs of W <= 12
-                code = build(false, true);
-                if (code) return raise(code, func, err.c_str());
-                s.plannedFns.assign(s.planned.size(), nullptr);
-            }
+            // the interpreting kernel runs unpaired programs of W <= 12, with
+            // diagonal gates where it spends least on them
+            code = build(false, true);
+            if (code) return raise(code, func, err.c_str());
+            s.plannedFns.assign(s.planned.size(), nullptr);
         } else {
             dgq::JitStats js;
             std::string jerr;

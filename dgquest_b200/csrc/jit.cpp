@@ -747,6 +747,8 @@ std::string generatePairedSource(const TileProgram &prog, int W) {
         }
         if (gPhase < 0 && nPhaseOps[p] > 0 && (prog.renormIn || prog.hasGlobal)) gPhase = p;
     }
+    for (int p = 0; p < np && gPhase < 0; p++)
+        if (nSignOps[p] > 0 && (prog.renormIn || prog.hasGlobal)) gPhase = p;
     if (firstDirect) {
         emitPairedLayoutAddressing(o, prog.phases[0], W, "gIn", "rbIn");
         o << "#pragma unroll\n    for (int j = 0; j < dgq::kRegs; j++) { const uint64_t g_ = dgq::jIdx(gIn, rbIn, j); "
@@ -848,14 +850,16 @@ std::string generateSweepSource(const TileProgram &prog, int W) {
     // the sweep's global factor (and renormalisation) is one number for all
     // amplitudes: it starts the factor of the first phase with a scalar
     // phase op instead of costing a multiply of its own at the end
+    // (with no such op, the factor of the first phase with a scalar sign flip)
     int gPhase = -1;
     if (prog.renormIn || prog.hasGlobal)
-        for (int p = 0; p < np && gPhase < 0; p++)
-            for (int k = prog.phases[p].opBegin; k < prog.phases[p].opEnd; k++)
-                if (scalarKind(prog.ops[k]) == 1) {
-                    gPhase = p;
-                    break;
-                }
+        for (int kind = 1; kind <= 2 && gPhase < 0; kind++)
+            for (int p = 0; p < np && gPhase < 0; p++)
+                for (int k = prog.phases[p].opBegin; k < prog.phases[p].opEnd; k++)
+                    if (scalarKind(prog.ops[k]) == kind) {
+                        gPhase = p;
+                        break;
+                    }
     if (firstDirect) {
         emitDirectAddressing(o, prog.phases[0], W, "gIn", "rbIn");
         o << "    dgq::jLoadDirect<" << prog.initKind << ", " << (prog.hasRestrict ? "true" : "false")

@@ -23,6 +23,7 @@ namespace dgq {
 struct BlockPlan {
     u64 tileMask = 0;         // W address bits, bits 0..4 always included
     std::vector<Gate> gates;  // dependency order
+    bool last = true;         // no gates are left after this block
 };
 
 struct PlanStats {
@@ -72,9 +73,14 @@ struct SweepHeader {
 
 // paired: encode for the complex64 paired form (TileProgram::paired); fails
 // (with *err set) on a multi-qubit unitary that targets address bit 0.
+// folds: the program is for a specialised kernel, which folds phase factors
+// on thread bits into one factor per thread; diagonal gates then move to the
+// phases where they are such factors. carry (with folds): diagonal gates of
+// the block before, run first here; the block's own that would be cheaper in
+// the next block are left in it (none when the block is the last).
 bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits, const MatrixPool &pool,
                  const SweepHeader &first, std::vector<TileProgram> &out, PlanStats *stats, std::string *err,
-                 bool paired = false);
+                 bool paired = false, bool folds = false, std::vector<Gate> *carry = nullptr);
 
 // A program that only applies the header (init and/or lazy collapse).
 void encodeHeaderOnly(int numBits, int numReal, int tileBits, const SweepHeader &hdr, TileProgram &out,

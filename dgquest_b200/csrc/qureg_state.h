@@ -124,7 +124,7 @@ namespace dgq {
 // complete, in order; when it returns false, planning stops and
 // buildPrograms returns -1 (the callback has reported its own error).
 int buildPrograms(QuregState &s, int W, std::vector<TileProgram> &out, PlanStats &st, std::string &err,
-                  bool paired = false, const std::function<bool(size_t)> &emit = nullptr);
+                  bool paired = false, const std::function<bool(size_t)> &emit = nullptr, bool folds = false);
 // Drops the pending work that buildPrograms planned (after it has been
 // launched or kept for launching).
 void consumePending(QuregState &s);
