@@ -32,7 +32,32 @@ const char *kernelKindName(int code) {
     return "jZ2R";
 }
 
-void emitOp(std::ostringstream &o, const KOp &op) {
+// The entries of a dense op's matrix that take part, as a type for jDenseAt:
+// re(i) / im(i) whether the part of entry i is non-zero, same(r) whether row r
+// is exactly a row of the identity. `m`: the coefficients, 2^k x 2^k (re, im).
+std::string densePattern(const double *m, int k) {
+    const int D = 1 << k;
+    uint64_t re[4] = {0}, im[4] = {0};
+    unsigned same = 0;
+    for (int r = 0; r < D; r++) {
+        bool identity = true;
+        for (int c = 0; c < D; c++) {
+            const int i = r * D + c;
+            if (m[2 * i] != 0.0) re[i >> 6] |= 1ULL << (i & 63);
+            if (m[2 * i + 1] != 0.0) im[i >> 6] |= 1ULL << (i & 63);
+            identity = identity && m[2 * i] == (r == c ? 1.0 : 0.0) && m[2 * i + 1] == 0.0;
+        }
+        if (identity) same |= 1u << r;
+    }
+    std::ostringstream o;
+    o << "dgq::DensePattern<";
+    for (uint64_t w : re) o << w << "ull, ";
+    for (uint64_t w : im) o << w << "ull, ";
+    o << same << "u>";
+    return o.str();
+}
+
+void emitOp(std::ostringstream &o, const KOp &op, const double *coefs) {
     const unsigned cr = op.ctrlReg;
     const int off = op.coef;
     std::ostringstream body;
@@ -71,7 +96,12 @@ void emitOp(std::ostringstream &o, const KOp &op) {
     } else if (op.code == KC_MULNI || op.code == KC_MULNI + 1) {
         body << "dgq::jMULNI<" << (op.code == KC_MULNI + 1 ? "true" : "false") << ", " << cr << "u>(a);";
     } else if (op.code >= KC_DENSE && op.code < KC_DENSE + 4) {
-        body << "dgq::jDense<" << (op.code - KC_DENSE + 1) << ", " << cr << "u>(a, prog.coef + " << off << ");";
+        const int k = op.code - KC_DENSE + 1;
+        if (op.selLoc & kDenseAnyBits)
+            body << "dgq::jDenseAt<" << k << ", " << (op.selLoc & 0xFF) << "u, " << densePattern(coefs + off, k)
+                 << ">(a, prog.coef + " << off << ");";
+        else
+            body << "dgq::jDense<" << k << ", " << cr << "u>(a, prog.coef + " << off << ");";
     } else if (op.code >= KC_RY1 && op.code < KC_H1) {
         static const char *names[4] = {"jRY1", "jRY2", "jRX1", "jRX2"};
         body << "dgq::" << names[(op.code - KC_RY1) / 4] << "<" << (op.code - KC_RY1) % 4 << ">(a, prog.coef + " << off
@@ -890,7 +920,7 @@ std::string generateSweepSource(const TileProgram &prog, int W) {
             if (fold && scalarKind(prog.ops[k]))
                 emitScalarAcc(o, prog.ops[k]);
             else
-                emitOp(o, prog.ops[k]);
+                emitOp(o, prog.ops[k], prog.coef);
         }
         if (fold) o << "    dgq::jGlobal(a, acc_.x, acc_.y);\n";
         if (writeSmem) {

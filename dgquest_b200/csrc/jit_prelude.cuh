@@ -296,6 +296,61 @@ __device__ __forceinline__ void jDense(V (&a)[kRegs], const double *m) {
     }
 }
 
+// Which entries of a dense op's matrix take part (words of 64 entries, row-major).
+template <uint64_t R0, uint64_t R1, uint64_t R2, uint64_t R3, uint64_t I0, uint64_t I1, uint64_t I2, uint64_t I3,
+          uint32_t SAME>
+struct DensePattern {
+    static __device__ __forceinline__ constexpr bool at(uint64_t w0, uint64_t w1, uint64_t w2, uint64_t w3, int i) {
+        return (((i >> 6) == 0 ? w0 : (i >> 6) == 1 ? w1 : (i >> 6) == 2 ? w2 : w3) >> (i & 63)) & 1u;
+    }
+    static __device__ __forceinline__ constexpr bool re(int i) { return at(R0, R1, R2, R3, i); }
+    static __device__ __forceinline__ constexpr bool im(int i) { return at(I0, I1, I2, I3, i); }
+    static __device__ __forceinline__ constexpr bool same(int r) { return (SAME >> r) & 1u; }
+};
+
+// Dense op with matrix bit i on register bit (POS >> 2 i) & 3, only the
+// entries of pattern M: a depolarising or damping channel's 4 x 4
+// superoperator has 6 real entries (48 FP64 instructions a thread instead of
+// 256), a two-qubit one 28 of 256.
+template <int KK, uint32_t POS, class M, class V>
+__device__ __forceinline__ void jDenseAt(V (&a)[kRegs], const double *m) {
+    constexpr int D = 1 << KK;
+    constexpr int b0 = 1 << (POS & 3), b1 = KK > 1 ? 1 << ((POS >> 2) & 3) : 0,
+                  b2 = KK > 2 ? 1 << ((POS >> 4) & 3) : 0, b3 = KK > 3 ? 1 << ((POS >> 6) & 3) : 0;
+    constexpr int mask = b0 | b1 | b2 | b3;
+#pragma unroll
+    for (int base = 0; base < kRegs; base++) {
+        if (base & mask) continue;
+        V v[D];
+#pragma unroll
+        for (int c = 0; c < D; c++)
+            v[c] = a[base | ((c & 1) ? b0 : 0) | ((c & 2) ? b1 : 0) | ((c & 4) ? b2 : 0) | ((c & 8) ? b3 : 0)];
+#pragma unroll
+        for (int r = 0; r < D; r++) {
+            if (M::same(r)) continue;
+            DGQJ_R re = 0, im = 0;
+            bool some = false;
+#pragma unroll
+            for (int c = 0; c < D; c++) {
+                const int i = r * D + c;
+                if (M::re(i)) {
+                    const DGQJ_R k = (DGQJ_R) m[2 * i];
+                    re = some ? fma(k, v[c].x, re) : k * v[c].x;
+                    im = some ? fma(k, v[c].y, im) : k * v[c].y;
+                    some = true;
+                }
+                if (M::im(i)) {
+                    const DGQJ_R k = (DGQJ_R) m[2 * i + 1];
+                    re = some ? fma(-k, v[c].y, re) : -k * v[c].y;
+                    im = some ? fma(k, v[c].x, im) : k * v[c].x;
+                    some = true;
+                }
+            }
+            a[base | ((r & 1) ? b0 : 0) | ((r & 2) ? b1 : 0) | ((r & 4) ? b2 : 0) | ((r & 8) ? b3 : 0)] = DGQJ_MK(re, im);
+        }
+    }
+}
+
 // ---------------------------------------------------------------- tile I/O
 // Canonical element (tid, j) of the tile sits at tile-local index
 // tid + T * j: lanes cover the 5 lowest address bits, j the top 4 tile bits.

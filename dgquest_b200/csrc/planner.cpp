@@ -480,7 +480,11 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
                 if (err) *err = "a gate has more non-diagonal targets than the register tile holds";
                 return false;
             }
-            // a dense multi-qubit gate fixes the register order: give it its own phase
+            // the interpreting kernels' (and the paired form's) dense op acts on
+            // register bits 0..k-1, so the gate fixes the register order and has
+            // a phase of its own; a specialised kernel takes any register bits
+            // (12-qubit density matrix, two layers with a channel per qubit: some
+            // 45 phases become 21, 2.19 -> 1.50 ms)
             Phase cur;
             auto flush = [&]() {
                 if (!cur.gates.empty()) phases.push_back(cur);
@@ -491,6 +495,11 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
                     if (paired && (g.targetMask & 1ULL)) {
                         if (err) *err = "paired form: a multi-qubit unitary targets address bit 0";
                         return false;
+                    }
+                    if (folds && !paired) {
+                        cur.gates.push_back(g);
+                        cur.targetsLocal |= splitMask(g.targetMask, tm).tileLocal;
+                        continue;
                     }
                     flush();
                     Phase d;
@@ -633,6 +642,12 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
                 op.k = (uint8_t) g.numMultiTargets;
                 const auto &m = pool.mats[(size_t) g.multiIndex];
                 coef.insert(coef.end(), m.begin(), m.end());
+                if (folds && !paired) {
+                    op.selLoc = kDenseAnyBits;
+                    for (int i = 0; i < g.numMultiTargets; i++)
+                        for (int b = 0; b < kRegBits; b++)
+                            if (L.regPos[b] == tm.local[g.multiTargets[i]]) op.selLoc |= (uint16_t) (b << (2 * i));
+                }
             } else {
                 const int k = targetReg(g.targetMask);
                 if (k < 0) {

@@ -45,7 +45,8 @@ enum KOpKind : uint8_t {
     KOP_MULNI = 8, // multiply by -i
     KOP_PH = 9,    // multiply by (c + i s)
     KOP_Z2 = 10,   // multiply by (c - i s) when the selector bit is 0, (c + i s) when 1
-    KOP_DENSE = 11, // dense 2^k x 2^k on register bits 0..k-1 (k = op.k), coefficients re/im
+    KOP_DENSE = 11, // dense 2^k x 2^k on register bits 0..k-1 (k = op.k), coefficients re/im; with
+                    // selLoc & kDenseAnyBits, matrix bit i on register bit (selLoc >> 2 i) & 3
     // Uncontrolled gates with their scalar factor moved into the sweep's
     // global factor (TileProgram::globalRe/Im), leaving unit entries:
     KOP_RY1 = 12,  // [[1, -t], [t, 1]]        (Ry with |cos| >= |sin|, t = tan)
@@ -63,6 +64,8 @@ enum KOpKind : uint8_t {
 constexpr uint32_t kLeanKinds = (1u << KOP_X) | (1u << KOP_NEG) | (1u << KOP_PH) | (1u << KOP_Z2) |
                                 (1u << KOP_RY1) | (1u << KOP_RY2) | (1u << KOP_RX1) | (1u << KOP_RX2) |
                                 (1u << KOP_H1) | (1u << KOP_PH1);
+
+constexpr uint16_t kDenseAnyBits = 0x8000;
 
 // Dispatch codes of the tile kernel: one straight-line case per
 // (operation, target register bit, register-control present). Pair
