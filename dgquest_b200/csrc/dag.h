@@ -57,32 +57,41 @@ public:
         flatValid_ = false;
     }
 
+    // countAllowed for each of n sets, in one scan for every 8.
+    void countAllowed(const u64 *allowed, size_t n, size_t *counts) const;
+
 private:
     // Alive nodes in insertion order as (touched qubits, non-diagonal
     // targets): a gate can run inside `allowed` exactly when its targets lie
     // in `allowed` and no earlier gate on one of its qubits was held back,
     // because its predecessors are the latest earlier gates on its qubits.
-    // The scans below run over this flat copy, rebuilt after a change.
+    // The queries and takeAllowed scan this flat copy, rebuilt after a change.
     void refreshFlat() const;
     mutable bool flatValid_ = false;
     bool touchCost_ = false;
     mutable std::vector<u64> flatTouch_, flatCost_;
+    mutable std::vector<int> flatNode_;
 
     struct Node {
         Gate g;
-        std::vector<int> prev;
-        std::vector<int> next;
+        int prevBegin = 0, prevCount = 0;  // in prevPool_: the latest earlier gates on its qubits
+        int next = 0;                      // alive gates that have this one among those
         bool alive = true;
     };
     bool tryMerge(int top, const Gate &g);
     void unlinkDeleted(int idx);
+    void rebuild();
 
     int numQubits_;
     bool merge_;
     size_t alive_ = 0;
     std::vector<Node> nodes_;
+    std::vector<int> prevPool_;
     std::vector<std::vector<int>> qubitStack_;
-    std::vector<int> front_;
+    // a gate became a general unitary by merging: added again after the gates
+    // before it are taken, it can absorb the gate that was before it
+    bool remerge_ = false;
+    bool stale_ = false;  // gates were taken since the links were made
 };
 
 // Product of two 2x2 complex matrices (row-major re/im): c = a * b.

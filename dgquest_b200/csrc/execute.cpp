@@ -214,10 +214,10 @@ double predictDenseSeconds(const QuregState &s, int K, int *blocksOut, double bo
     const CostModel cm = costModel();
     const double perBlock = denseSweepSeconds(s, K, cm);
     const int maxBlocks = bound > 0.0 ? (int) std::min(1e6, std::floor(bound / perBlock)) + 1 : 0;
-    dgq::MatrixPool pool = s.pool;
+    dgq::MatrixPool none;
     int blocks = 0;
     bool cut = false;
-    const std::vector<Gate> fused = dgq::fuseDenseBlocks(s.pending, s.numBits, K, pool, &blocks, maxBlocks, &cut);
+    const std::vector<Gate> fused = dgq::fuseDenseBlocks(s.pending, s.numBits, K, none, &blocks, maxBlocks, &cut, false);
     if (blocksOut) *blocksOut = blocks;
     if (stopped) *stopped = cut;
     double t = blocks * perBlock;
@@ -226,7 +226,7 @@ double predictDenseSeconds(const QuregState &s, int K, int *blocksOut, double bo
     for (const Gate &g : fused)
         if (!isWide(g)) rest.push_back(g);
     if (!rest.empty()) {
-        const double tt = predictPlanSeconds(rest, s.numBits, std::min(12, s.numBits), pool, -1);
+        const double tt = predictPlanSeconds(rest, s.numBits, std::min(12, s.numBits), s.pool, -1);
         t += s.single ? tt * cm.c64TileFactor : tt;
     }
     return t + wideSeconds(s, fused, K, cm);
@@ -253,8 +253,13 @@ std::unordered_map<uint64_t, FormChoice> g_formCache;
 uint64_t formKey(const QuregState &s, const CostModel &cm) {
     uint64_t h = 1469598103934665603ULL;
     auto mix = [&](const void *p, size_t n) {
-        const unsigned char *b = static_cast<const unsigned char *>(p);
-        for (size_t i = 0; i < n; i++) h = (h ^ b[i]) * 1099511628211ULL;
+        const char *b = static_cast<const char *>(p);
+        for (size_t i = 0; i < n; i += 8) {
+            uint64_t w = 0;
+            std::memcpy(&w, b + i, std::min<size_t>(8, n - i));
+            h = (h ^ w) * 0x9E3779B97F4A7C15ULL;
+            h ^= h >> 29;
+        }
     };
     const int32_t shape[5] = {s.numBits, s.single ? 1 : 0, s.tileBitsSetting, g_tensorCores.load(),
                               (int32_t) s.pending.size()};
@@ -635,7 +640,12 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
                 setRenorm(s, i, SIZE_MAX, event);
                 CUfunction fn = nullptr;
                 if (wantJit && !s.planned[i].denseK) {
-                    fn = dgq::jitFindLoaded(dgq::generateSweepSource(s.planned[i], W));
+                    const std::string key = dgq::sweepKey(s.planned[i], W);
+                    fn = dgq::jitFindKey(key);
+                    if (!fn) {
+                        fn = dgq::jitFindLoaded(dgq::generateSweepSource(s.planned[i], W));
+                        dgq::jitRemember(key, fn);
+                    }
                     if (!fn) {
                         missing = true;
                         break;
@@ -684,11 +694,18 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
     s.stats.jitReused = reused;
     s.stats.jitMillis = 0.0;
     if (specialise && wantJit) {
-        std::vector<std::string> sources;
+        std::vector<std::string> sources, keys;
         std::vector<size_t> which;  // tile programs (dense sweeps have their own kernel)
+        int known = 0;
         for (size_t i = launched; i < s.planned.size(); i++)
             if (!s.planned[i].denseK) {
+                std::string key = dgq::sweepKey(s.planned[i], W);
+                if ((s.plannedFns[i] = dgq::jitFindKey(key))) {
+                    known++;
+                    continue;
+                }
                 sources.push_back(dgq::generateSweepSource(s.planned[i], W));
+                keys.push_back(std::move(key));
                 which.push_back(i);
             }
         if (cachedOnly && !dgq::jitAllReady(sources)) {
@@ -703,9 +720,12 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
             std::string jerr;
             std::vector<CUfunction> fns;
             if (!dgq::jitGetKernels(sources, fns, &js, &jerr)) return raise(E_UNSUPPORTED, func, jerr.c_str());
-            for (size_t k = 0; k < which.size(); k++) s.plannedFns[which[k]] = fns[k];
+            for (size_t k = 0; k < which.size(); k++) {
+                s.plannedFns[which[k]] = fns[k];
+                dgq::jitRemember(keys[k], fns[k]);
+            }
             s.stats.jitCompiled = js.compiled;
-            s.stats.jitReused += js.reused;
+            s.stats.jitReused += js.reused + known;
             s.stats.jitMillis = js.compileMillis;
         }
     }

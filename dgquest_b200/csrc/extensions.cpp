@@ -468,6 +468,13 @@ int dgq_setSpecialisationMinBits(int minBits) {
 int dgq_sweepSource(int numQubits, int tileBits, int count, const int32_t *types, const uint64_t *targetMasks,
                     const uint64_t *controlMasks, const double *operands, int sweep, int precision, char *buf,
                     int len) {
+    return dgq_sweepSourceKey(numQubits, tileBits, count, types, targetMasks, controlMasks, operands, sweep, precision,
+                              buf, len, nullptr);
+}
+
+int dgq_sweepSourceKey(int numQubits, int tileBits, int count, const int32_t *types, const uint64_t *targetMasks,
+                       const uint64_t *controlMasks, const double *operands, int sweep, int precision, char *buf,
+                       int len, uint64_t *keyHash) {
     if (numQubits < 1 || numQubits > dgq::kMaxStateBits - 2 || count < 0 || !buf || len <= 0) {
         raise(E_INVALID_ARGUMENT, __func__);
         return -1;
@@ -491,6 +498,7 @@ int dgq_sweepSource(int numQubits, int tileBits, int count, const int32_t *types
     if (!ok) return -1;
     if (sweep < 0 || sweep >= (int) s.planned.size()) return (int) s.planned.size();
     const std::string src = dgq::generateSweepSource(s.planned[(size_t) sweep], s.plannedTileBits);
+    if (keyHash) *keyHash = std::hash<std::string>()(dgq::sweepKey(s.planned[(size_t) sweep], s.plannedTileBits));
     std::strncpy(buf, src.c_str(), (size_t) len - 1);
     buf[len - 1] = '\0';
     return (int) src.size() < len ? (int) s.planned.size() : -2;

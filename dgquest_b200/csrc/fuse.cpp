@@ -117,7 +117,7 @@ void applyGateLocal(const Gate &g, const MatrixPool &pool, const int local[64], 
 }
 
 std::vector<Gate> fuseDenseBlocks(const std::vector<Gate> &gates, int numBits, int K, MatrixPool &pool,
-                                  int *blocks, int maxBlocks, bool *stopped) {
+                                  int *blocks, int maxBlocks, bool *stopped, bool compose) {
     std::vector<Gate> out;
     if (blocks) *blocks = 0;
     if (stopped) *stopped = false;
@@ -128,6 +128,8 @@ std::vector<Gate> fuseDenseBlocks(const std::vector<Gate> &gates, int numBits, i
     for (const Gate &g : gates) dag.add(g);
     const int D = 1 << K;
     std::vector<double> u((size_t) 2 * D * D);
+    std::vector<u64> adds, sets;
+    std::vector<size_t> counts;
     while (!dag.empty()) {
         if (maxBlocks > 0 && made >= maxBlocks) {
             if (stopped) *stopped = true;
@@ -137,9 +139,18 @@ std::vector<Gate> fuseDenseBlocks(const std::vector<Gate> &gates, int numBits, i
         for (;;) {
             size_t best = 0;
             u64 bestAdd = 0;
-            for (u64 add : dag.frontierSets(mask)) {
-                if (__builtin_popcountll(mask | add) > K) continue;
-                const size_t c = dag.countAllowed(mask | add);
+            adds.clear();
+            sets.clear();
+            for (u64 add : dag.frontierSets(mask))
+                if (__builtin_popcountll(mask | add) <= K) {
+                    adds.push_back(add);
+                    sets.push_back(mask | add);
+                }
+            counts.resize(sets.size());
+            dag.countAllowed(sets.data(), sets.size(), counts.data());
+            for (size_t i = 0; i < adds.size(); i++) {
+                const u64 add = adds[i];
+                const size_t c = counts[i];
                 if (c > best || (c == best && bestAdd && __builtin_popcountll(add) < __builtin_popcountll(bestAdd))) {
                     best = c;
                     bestAdd = add;
@@ -175,6 +186,12 @@ std::vector<Gate> fuseDenseBlocks(const std::vector<Gate> &gates, int numBits, i
                 f.multiTargets[n++] = b;
             }
         }
+        made++;
+        if (blocks) (*blocks)++;
+        if (!compose) {
+            out.push_back(f);
+            continue;
+        }
         // columns of the identity, then every gate of the block in order
         std::fill(u.begin(), u.end(), 0.0);
         for (int c = 0; c < D; c++) u[(size_t) 2 * (c * D + c)] = 1.0;
@@ -189,8 +206,6 @@ std::vector<Gate> fuseDenseBlocks(const std::vector<Gate> &gates, int numBits, i
         f.multiIndex = (int32_t) pool.mats.size();
         pool.mats.push_back(std::move(m));
         out.push_back(f);
-        made++;
-        if (blocks) (*blocks)++;
     }
     return out;
 }

@@ -25,9 +25,11 @@ namespace dgq {
 // Requires 1 <= K <= 7 and K <= numBits.
 // maxBlocks > 0 stops after that many blocks (the rest of the gates are
 // dropped; *stopped, if given, is set): a cost estimate that only needs to
-// know whether the form stays below a bound.
+// know whether the form stays below a bound. compose = false leaves the
+// matrices out (the gates have no multiIndex): for estimates too.
 std::vector<Gate> fuseDenseBlocks(const std::vector<Gate> &gates, int numBits, int K, MatrixPool &pool,
-                                  int *blocks = nullptr, int maxBlocks = 0, bool *stopped = nullptr);
+                                  int *blocks = nullptr, int maxBlocks = 0, bool *stopped = nullptr,
+                                  bool compose = true);
 
 // Applies one recorded gate to the 2^K-amplitude vectors v[c * 2^K ..] for
 // c < numVectors, where local[b] is the vector index bit of address bit b

@@ -947,6 +947,23 @@ std::string generateSweepSource(const TileProgram &prog, int W) {
     return o.str();
 }
 
+std::string sweepKey(const TileProgram &prog, int W) {
+    // the phases and ops whole, and the header fields that choose code; the
+    // other fields and the coefficients are read at run time, except for
+    // which entries of a dense op on any register bits are zero
+    const int32_t head[10] = {W,         prog.numPhases, prog.numOps,   prog.initKind,  prog.hasRestrict != 0,
+                              prog.hasGlobal, prog.isSingle,  prog.renormIn, prog.renormOut, prog.paired};
+    std::string key;
+    key.reserve(sizeof(head) + (size_t) prog.numPhases * sizeof(KPhase) + (size_t) prog.numOps * sizeof(KOp));
+    key.append(reinterpret_cast<const char *>(head), sizeof(head));
+    key.append(reinterpret_cast<const char *>(prog.phases), (size_t) prog.numPhases * sizeof(KPhase));
+    key.append(reinterpret_cast<const char *>(prog.ops), (size_t) prog.numOps * sizeof(KOp));
+    for (int i = 0; i < prog.numOps; i++)
+        if (prog.ops[i].kind == KOP_DENSE && (prog.ops[i].selLoc & kDenseAnyBits))
+            key += densePattern(prog.coef + prog.ops[i].coef, prog.ops[i].k);
+    return key;
+}
+
 bool jitEnabled() {
     static int enabled = -1;
     if (enabled < 0) {
@@ -1030,6 +1047,12 @@ CUfunction cacheFind(const std::string &src) {
         if (e.device == dev && e.source == src) return e.fn;
     return nullptr;
 }
+
+// Kernels by program key and device; they are never unloaded. Cleared when it
+// grows beyond what a program's working set of structures can be.
+std::mutex g_keyMutex;
+std::unordered_map<std::string, CUfunction> g_keys;
+constexpr size_t kMaxKeys = 16384;
 
 bool compileOne(const std::string &src, std::vector<char> &cubin, std::string &log) {
     nvrtcProgram prog;
@@ -1125,6 +1148,23 @@ void backgroundWorker() {
 }
 
 }  // namespace
+
+CUfunction jitFindKey(const std::string &key) {
+    std::string k = key;
+    k += (char) currentDevice();
+    std::lock_guard<std::mutex> lk(g_keyMutex);
+    auto it = g_keys.find(k);
+    return it == g_keys.end() ? nullptr : it->second;
+}
+
+void jitRemember(const std::string &key, CUfunction fn) {
+    if (!fn) return;
+    std::string k = key;
+    k += (char) currentDevice();
+    std::lock_guard<std::mutex> lk(g_keyMutex);
+    if (g_keys.size() >= kMaxKeys) g_keys.clear();
+    g_keys[k] = fn;
+}
 
 CUfunction jitFindLoaded(const std::string &source) { return cacheFind(source); }
 

@@ -20,6 +20,13 @@ namespace dgq {
 
 std::string generateSweepSource(const TileProgram &prog, int tileBits);
 
+// Everything of a program that its source depends on: programs of equal keys
+// have equal sources. A key takes a microsecond, a source 30..60.
+std::string sweepKey(const TileProgram &prog, int tileBits);
+// The kernel remembered for a key on the current device, or nullptr.
+CUfunction jitFindKey(const std::string &key);
+void jitRemember(const std::string &key, CUfunction fn);
+
 struct JitStats {
     int compiled = 0;       // kernels compiled by the last call
     int reused = 0;         // kernels found in the cache by the last call

@@ -39,21 +39,39 @@ bool lookaheadBySize(int numBits) { return numBits >= lookaheadMinBits(); }
 // lookahead: score each candidate addition by the best follow-up addition too
 static void growMask(const GateDag &dag, u64 &mask, int budget, bool preferHigh, bool lookahead = false) {
     const u64 low = (1ULL << kCoalescedBits) - 1;
-    const bool look = lookahead;
+    std::vector<u64> sets;
+    std::vector<size_t> counts, score;
+    std::vector<std::pair<size_t, size_t>> uses;  // candidate, set
     while (popcount64(mask) < budget) {
-        const std::vector<u64> cands = dag.frontierSets(mask);
+        std::vector<u64> cands = dag.frontierSets(mask);
+        cands.erase(std::remove_if(cands.begin(), cands.end(),
+                                   [&](u64 add) { return popcount64(mask | add) > budget; }),
+                    cands.end());
+        // every candidate, and with lookahead every candidate with each
+        // follow-up addition (most unions come up from both sides): counted
+        // together
+        sets.clear();
+        uses.clear();
+        auto use = [&](size_t cand, u64 set) {
+            const size_t k = (size_t) (std::find(sets.begin(), sets.end(), set) - sets.begin());
+            if (k == sets.size()) sets.push_back(set);
+            uses.emplace_back(cand, k);
+        };
+        for (size_t i = 0; i < cands.size(); i++) {
+            use(i, mask | cands[i]);
+            if (lookahead && popcount64(mask | cands[i]) < budget)
+                for (u64 add2 : dag.frontierSets(mask | cands[i]))
+                    if (popcount64(mask | cands[i] | add2) <= budget) use(i, mask | cands[i] | add2);
+        }
+        counts.resize(sets.size());
+        dag.countAllowed(sets.data(), sets.size(), counts.data());
+        score.assign(cands.size(), 0);
+        for (const auto &u : uses) score[u.first] = std::max(score[u.first], counts[u.second]);
         size_t best = 0;
         u64 bestAdd = 0;
-        for (u64 add : cands) {
-            if (popcount64(mask | add) > budget) continue;
-            size_t c = dag.countAllowed(mask | add);
-            if (look && popcount64(mask | add) < budget) {
-                // score a candidate by the best follow-up addition as well
-                for (u64 add2 : dag.frontierSets(mask | add)) {
-                    if (popcount64(mask | add | add2) > budget) continue;
-                    c = std::max(c, dag.countAllowed(mask | add | add2));
-                }
-            }
+        for (size_t i = 0; i < cands.size(); i++) {
+            const u64 add = cands[i];
+            const size_t c = score[i];
             bool better = c > best;
             if (!better && c == best && bestAdd) {
                 const int pa = popcount64(add), pb = popcount64(bestAdd);

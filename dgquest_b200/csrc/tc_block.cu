@@ -516,20 +516,28 @@ void packTcBlockMatrix(int K, const double *Uin, const uint8_t *targets, float *
     const uint32_t groups = (uint32_t) (2 * KR / 8);
     unsigned char *bytes = reinterpret_cast<unsigned char *>(out);
     std::memset(bytes, 0, (size_t) KR * 2 * KR * 2);
-    for (int n = 0; n < KR; n++)
-        for (int k = 0; k < KR; k++) {
-            const int so = n >> 1, ro = n & 1, si = k >> 1, ri = k & 1;
-            const double ur = U[2 * (so * D + si)], ui = U[2 * (so * D + si) + 1];
-            double w;
-            if (ro == 0)
-                w = ri == 0 ? ur : -ui;
-            else
-                w = ri == 0 ? ui : ur;
-            w *= (double) kTbWScale;
-            const __half hi = __double2half((double) w);
-            const __half lo = __double2half(w - (double) __half2float(hi));
-            std::memcpy(bytes + tbOffset((uint32_t) n, (uint32_t) k, groups), &hi, 2);
-            std::memcpy(bytes + tbOffset((uint32_t) (KR + n), (uint32_t) k, groups), &lo, 2);
+    // each part of an entry is split once and stored twice, the imaginary one
+    // negated for the real output (128 x 128 values of 64 x 64 entries)
+    auto put = [&](int n, int k, __half hi, __half lo) {
+        std::memcpy(bytes + tbOffset((uint32_t) n, (uint32_t) k, groups), &hi, 2);
+        std::memcpy(bytes + tbOffset((uint32_t) (KR + n), (uint32_t) k, groups), &lo, 2);
+    };
+    auto negated = [](__half h) {
+        uint16_t b;
+        std::memcpy(&b, &h, 2);
+        b ^= 0x8000u;
+        std::memcpy(&h, &b, 2);
+        return h;
+    };
+    for (int so = 0; so < D; so++)
+        for (int si = 0; si < D; si++) {
+            const double ur = U[2 * (so * D + si)] * (double) kTbWScale, ui = U[2 * (so * D + si) + 1] * (double) kTbWScale;
+            const __half rh = __double2half(ur), rl = __double2half(ur - (double) __half2float(rh));
+            const __half ih = __double2half(ui), il = __double2half(ui - (double) __half2float(ih));
+            put(2 * so, 2 * si, rh, rl);
+            put(2 * so, 2 * si + 1, negated(ih), negated(il));
+            put(2 * so + 1, 2 * si, ih, il);
+            put(2 * so + 1, 2 * si + 1, rh, rl);
         }
 }
 

@@ -216,6 +216,8 @@ _SIGS = {
     "dgq_getPrecision": (I, [Q]),
     "dgq_sweepSource": (I, [I, I, I, P(ctypes.c_int32), P(ctypes.c_uint64), P(ctypes.c_uint64), P(D), I, I,
                             ctypes.c_char_p, I]),
+    "dgq_sweepSourceKey": (I, [I, I, I, P(ctypes.c_int32), P(ctypes.c_uint64), P(ctypes.c_uint64), P(D), I, I,
+                            ctypes.c_char_p, I, P(ctypes.c_uint64)]),
     "dgq_compileSweepSource": (I, [ctypes.c_char_p, ctypes.c_char_p, I]),
     "dgq_specialiseGates": (I, [I, I, I, P(ctypes.c_int32), P(ctypes.c_uint64), P(ctypes.c_uint64), P(D), I]),
     "dgq_setSpecialisationMinBits": (I, [I]),

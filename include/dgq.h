@@ -266,6 +266,11 @@ int dgq_getDeviceErrors(void);
 int dgq_sweepSource(int numQubits, int tileBits, int count, const int32_t *types, const uint64_t *targetMasks,
                     const uint64_t *controlMasks, const double *operands, int sweep, int precision, char *buf,
                     int len);
+/* The same; *keyHash (if not NULL) receives a hash of the key under which the
+ * sweep's loaded kernel is found (equal keys: equal sources). */
+int dgq_sweepSourceKey(int numQubits, int tileBits, int count, const int32_t *types, const uint64_t *targetMasks,
+                       const uint64_t *controlMasks, const double *operands, int sweep, int precision, char *buf,
+                       int len, uint64_t *keyHash);
 int dgq_compileSweepSource(const char *source, char *log, int len);
 
 /* Compiles ahead of time the specialised sweep kernels that a register of
