@@ -14,6 +14,7 @@
 #include <cstring>
 
 #include "batch.h"
+#include "frame.cuh"
 #include "interp.cuh"
 #include "tile_program.h"
 
@@ -95,7 +96,7 @@ __device__ __noinline__ void addExpectationSums(double tot, const double (&rs)[4
 
 // One tile of one sweep, run by the first 2^(W-4) threads of the CTA; h is
 // the sweep header staged in shared memory.
-template <class V, int W, bool DENSE, bool LEAN>
+template <class V, int W, int FORM>
 __device__ __forceinline__ void sweepTile(const BatchArgs &args, const BatchSweep &h, V *__restrict__ st, uint32_t tile,
                                           V *sm, double *zs) {
     constexpr uint32_t T = 1u << (W - kRegBits);
@@ -143,45 +144,55 @@ __device__ __forceinline__ void sweepTile(const BatchArgs &args, const BatchSwee
         }
     }
 
-    const KPhase *phases = args.phases + h.phaseOff;
-    const KOp *__restrict__ ops = args.ops + h.opOff;
-    const double *__restrict__ coef = args.coef + h.coefOff;
     if (h.numPhases > 0) {
 #pragma unroll
         for (int j = 0; j < kRegs; j++) sm[swzB(tid + T * (uint32_t) j)] = a[j];
         groupBarrier(T);
-        for (int p = 0; p < h.numPhases; p++) {
-            const KPhase &ph = phases[p];
-            uint32_t loc = 0;
+        if constexpr (FORM == kBatchFormFramed) {
+            const FPhase *phases = args.framePhases + h.phaseOff;
+            const FOp *__restrict__ ops = args.frameOps + h.opOff;
+            const double2 *__restrict__ coef = args.frameCoef + h.opOff;
+            framePhases<V, W>(
+                h.numPhases, h.tail, sm, tid, tile, [&](int p) -> const FPhase & { return phases[p]; },
+                [&](int o) {
+                    // the 16-byte op record in one read-only load
+                    const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(ops + o));
+                    FOp op;
+                    memcpy(&op, &raw, sizeof(op));
+                    return op;
+                },
+                [&](int o) { return __ldg(coef + o); }, [] { groupBarrier(T); });
+        } else {
+            const KPhase *phases = args.phases + h.phaseOff;
+            const KOp *__restrict__ ops = args.ops + h.opOff;
+            const double *__restrict__ coef = args.coef + h.coefOff;
+            for (int p = 0; p < h.numPhases; p++) {
+                const KPhase &ph = phases[p];
+                uint32_t loc = 0;
 #pragma unroll
-            for (int i = 0; i < W - kRegBits; i++) loc |= ((tid >> i) & 1u) << ph.thrPos[i];
-            const uint32_t sb = swzB(loc);
+                for (int i = 0; i < W - kRegBits; i++) loc |= ((tid >> i) & 1u) << ph.thrPos[i];
+                const uint32_t sb = swzB(loc);
 #pragma unroll
-            for (int j = 0; j < kRegs; j++) a[j] = sm[sb ^ ph.regOff[j]];
-            const int e = ph.opEnd;
-            for (int o = ph.opBegin; o < e; o++) {
-                // the 16-byte op record in one read-only load
-                const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(ops + o));
-                KOp op;
-                memcpy(&op, &raw, sizeof(op));
-                if constexpr (LEAN) {
-                    // the lean kinds' two coefficients, loaded beside the
-                    // record instead of after it
-                    const double2 cc = __ldg(args.leanCoef + h.opOff + o);
-                    const double cv[2] = {cc.x, cc.y};
-                    applyOpAt<V, DENSE, LEAN>(op, cv, a, loc, tile);
-                } else {
-                    applyOp<V, DENSE, LEAN>(op, coef, a, loc, tile);
+                for (int j = 0; j < kRegs; j++) a[j] = sm[sb ^ ph.regOff[j]];
+                const int e = ph.opEnd;
+                for (int o = ph.opBegin; o < e; o++) {
+                    // the 16-byte op record in one read-only load
+                    const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(ops + o));
+                    KOp op;
+                    memcpy(&op, &raw, sizeof(op));
+                    applyOp<V, FORM == kBatchFormDense>(op, coef, a, loc, tile);
                 }
-            }
 #pragma unroll
-            for (int j = 0; j < kRegs; j++) sm[sb ^ ph.regOff[j]] = a[j];
-            groupBarrier(T);
+                for (int j = 0; j < kRegs; j++) sm[sb ^ ph.regOff[j]] = a[j];
+                groupBarrier(T);
+            }
         }
 #pragma unroll
         for (int j = 0; j < kRegs; j++) a[j] = sm[swzB(tid + T * (uint32_t) j)];
     }
-    if (h.hasGlobal) {
+    if constexpr (FORM == kBatchFormFramed) {
+        frameFinish(h.tail, a, tid, tile, false, 1.0);
+    } else if (h.hasGlobal) {
         const typename Real<V>::T gr = (typename Real<V>::T) h.globalRe, gi = (typename Real<V>::T) h.globalIm;
 #pragma unroll
         for (int j = 0; j < kRegs; j++) a[j] = mk<V>(gr * a[j].x - gi * a[j].y, gr * a[j].y + gi * a[j].x);
@@ -219,7 +230,7 @@ __device__ __forceinline__ void sweepTile(const BatchArgs &args, const BatchSwee
 // Sweeps [w0, w1) of one register on tile `tile` (one sweep for a tile
 // item, all of them for a whole-register item); each header is copied to
 // shared memory first, so the phase loop holds no header registers.
-template <class V, int W, bool DENSE, bool LEAN>
+template <class V, int W, int FORM>
 __device__ __forceinline__ void runSweeps(const BatchArgs &args, const BatchCircuit &C, uint32_t w0, uint32_t w1,
                                        uint32_t tile, V *sm, BatchSweep *hs) {
     constexpr uint32_t T = 1u << (W - kRegBits);
@@ -229,15 +240,14 @@ __device__ __forceinline__ void runSweeps(const BatchArgs &args, const BatchCirc
         uint32_t *dst = reinterpret_cast<uint32_t *>(hs);
         for (uint32_t i = threadIdx.x; i < sizeof(BatchSweep) / 4; i += T) dst[i] = __ldg(src + i);
         groupBarrier(T);
-        sweepTile<V, W, DENSE, LEAN>(args, *hs, st, tile, sm, w + 1 == C.numSweeps ? args.zsum + C.zOff : nullptr);
+        sweepTile<V, W, FORM>(args, *hs, st, tile, sm, w + 1 == C.numSweeps ? args.zsum + C.zOff : nullptr);
     }
 }
 
-// DENSE: the batch's programs hold dense ops (multi-qubit unitaries of up to
-// 4 targets inside a register phase); without them the kernel is compiled
-// without that case (FP64: no spills instead of 1.3 KB of spill stores).
-// LEAN: every op kind is one of kLeanKinds (rotations, CNOT, CZ, phases).
-template <class V, bool DENSE, bool LEAN>
+// FORM: kBatchFormDense for programs with dense ops (multi-qubit unitaries of
+// up to 4 targets inside a register phase), whose case costs FP64 1.3 KB of
+// spill stores; kBatchFormGeneral; kBatchFormFramed.
+template <class V, int FORM>
 __global__ void __launch_bounds__(1 << (kBatchMaxTileBits - kRegBits), 2)
     batchKernel(const __grid_constant__ BatchArgs args) {
     extern __shared__ __align__(16) unsigned char smRaw[];
@@ -278,10 +288,10 @@ __global__ void __launch_bounds__(1 << (kBatchMaxTileBits - kRegBits), 2)
             const uint32_t w0 = s == kBatchWhole ? 0u : s, w1 = s == kBatchWhole ? C.numSweeps : s + 1;
             const uint32_t tile = s == kBatchWhole ? 0u : t;
             switch (C.tileBits) {
-                case 9: runSweeps<V, 9, DENSE, LEAN>(args, C, w0, w1, tile, sm, &sHead); break;
-                case 10: runSweeps<V, 10, DENSE, LEAN>(args, C, w0, w1, tile, sm, &sHead); break;
-                case 11: runSweeps<V, 11, DENSE, LEAN>(args, C, w0, w1, tile, sm, &sHead); break;
-                default: runSweeps<V, 12, DENSE, LEAN>(args, C, w0, w1, tile, sm, &sHead); break;
+                case 9: runSweeps<V, 9, FORM>(args, C, w0, w1, tile, sm, &sHead); break;
+                case 10: runSweeps<V, 10, FORM>(args, C, w0, w1, tile, sm, &sHead); break;
+                case 11: runSweeps<V, 11, FORM>(args, C, w0, w1, tile, sm, &sHead); break;
+                default: runSweeps<V, 12, FORM>(args, C, w0, w1, tile, sm, &sHead); break;
             }
             __threadfence();
         }
@@ -298,24 +308,24 @@ cudaError_t launchBatchV(const BatchArgs &a, int maxTileBits, int grid, int form
     const size_t smem = sizeof(V) << maxTileBits;
     const int T = 1 << (maxTileBits - kRegBits);
     if (form == kBatchFormDense)
-        batchKernel<V, true, false><<<grid, T, smem, s>>>(a);
-    else if (form == kBatchFormLean)
-        batchKernel<V, false, true><<<grid, T, smem, s>>>(a);
+        batchKernel<V, kBatchFormDense><<<grid, T, smem, s>>>(a);
+    else if (form == kBatchFormFramed)
+        batchKernel<V, kBatchFormFramed><<<grid, T, smem, s>>>(a);
     else
-        batchKernel<V, false, false><<<grid, T, smem, s>>>(a);
+        batchKernel<V, kBatchFormGeneral><<<grid, T, smem, s>>>(a);
     return cudaGetLastError();
 }
 
 // All forms have the same launch bounds and shared memory; the occupancy
 // is the smallest of them.
-template <class V, bool DENSE, bool LEAN>
+template <class V, int FORM>
 int ctasPerSmForm(int maxTileBits) {
     const size_t smem = sizeof(V) << maxTileBits;
-    if (cudaFuncSetAttribute(batchKernel<V, DENSE, LEAN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(batchKernel<V, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int) (sizeof(V) << kBatchMaxTileBits)) != cudaSuccess)
         return 0;
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batchKernel<V, DENSE, LEAN>, 1 << (maxTileBits - kRegBits),
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batchKernel<V, FORM>, 1 << (maxTileBits - kRegBits),
                                                       smem) != cudaSuccess)
         return 0;
     return n;
@@ -323,8 +333,8 @@ int ctasPerSmForm(int maxTileBits) {
 
 template <class V>
 int ctasPerSmV(int maxTileBits) {
-    const int a = ctasPerSmForm<V, true, false>(maxTileBits), b = ctasPerSmForm<V, false, false>(maxTileBits),
-              c = ctasPerSmForm<V, false, true>(maxTileBits);
+    const int a = ctasPerSmForm<V, kBatchFormDense>(maxTileBits), b = ctasPerSmForm<V, kBatchFormGeneral>(maxTileBits),
+              c = ctasPerSmForm<V, kBatchFormFramed>(maxTileBits);
     return std::min(a, std::min(b, c));
 }
 

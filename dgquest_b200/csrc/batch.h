@@ -20,6 +20,7 @@
 
 #include <cstdint>
 
+#include "frame.h"
 #include "tile_program.h"
 
 namespace dgq {
@@ -43,9 +44,10 @@ struct BatchSweep {
     double initAmp;
     uint64_t restrictMask, restrictValue;
     double restrictScale;
-    uint32_t phaseOff, opOff, coefOff, pad;
+    uint32_t phaseOff, opOff, coefOff, pad;  // framed form: of the framed arrays (coefficients go with the ops)
     uint8_t highPos[kMaxTileBits - kCoalescedBits];
     uint8_t ctaPos[kMaxStateBits];
+    FrameTail tail;  // framed form
 };
 
 struct BatchCircuit {
@@ -65,7 +67,10 @@ struct BatchArgs {
     const BatchSweep *sweeps;
     const KPhase *phases;
     const KOp *ops;
-    const double2 *leanCoef;  // lean form: the first two coefficients of each op, by op index
+    // framed form (frame.h); the phases and ops above are not used
+    const FPhase *framePhases;
+    const FOp *frameOps;
+    const double2 *frameCoef;  // two per op
     const double *coef;
     const uint64_t *items;  // c | s << 20 | t << 36
     uint32_t numItems;
@@ -84,9 +89,8 @@ inline uint64_t batchItem(uint32_t c, uint32_t s, uint32_t t) {
 // One launch of the persistent batch kernel: grid CTAs of 2^(maxTileBits-4)
 // threads with 2^maxTileBits amplitudes of shared memory.
 // Kernel forms: with the dense-op case (a program holds a dense op), the
-// general form, and the lean form (every op kind is a rotation, CNOT, CZ or
-// phase kind).
-constexpr int kBatchFormDense = 0, kBatchFormGeneral = 1, kBatchFormLean = 2;
+// general form, and the framed form (every program has one, frame.h).
+constexpr int kBatchFormDense = 0, kBatchFormGeneral = 1, kBatchFormFramed = 2;
 cudaError_t launchBatch(const BatchArgs &a, bool single, int maxTileBits, int grid, int form, cudaStream_t s);
 // CTAs of that kernel resident per SM (0 on error). Also sets the kernel's
 // shared-memory limit: call it before the first launch (and before a launch

@@ -58,6 +58,12 @@ struct RegPlan {
     std::vector<KPhase> phases;
     std::vector<KOp> ops;
     std::vector<double> coef;
+    // framed form (frame.h), when every sweep has one
+    bool framed = true;
+    std::vector<dgq::FPhase> framePhases;
+    std::vector<dgq::FOp> frameOps;
+    std::vector<double2> frameCoef;
+    std::vector<uint32_t> framePhaseOff, frameOpOff;  // per sweep
     double flopsPerAmp = 0.0;
     int err = 0;
     std::string errMsg;
@@ -88,6 +94,17 @@ void compact(const std::vector<TileProgram> &progs, int W, RegPlan &out) {
         h.coefOff = (uint32_t) out.coef.size();
         std::memcpy(h.highPos, p.highPos, sizeof(h.highPos));
         std::memcpy(h.ctaPos, p.ctaPos, sizeof(h.ctaPos));
+        dgq::FrameSweep f;
+        if (out.framed && dgq::frameProgram(p, W, f)) {
+            h.tail = f.tail;
+            out.framePhaseOff.push_back((uint32_t) out.framePhases.size());
+            out.frameOpOff.push_back((uint32_t) out.frameOps.size());
+            out.framePhases.insert(out.framePhases.end(), f.phases.begin(), f.phases.end());
+            out.frameOps.insert(out.frameOps.end(), f.ops.begin(), f.ops.end());
+            for (size_t o = 0; o < f.ops.size(); o++) out.frameCoef.push_back(make_double2(f.coef[2 * o], f.coef[2 * o + 1]));
+        } else {
+            out.framed = false;
+        }
         out.sweeps.push_back(h);
         out.phases.insert(out.phases.end(), p.phases, p.phases + p.numPhases);
         out.ops.insert(out.ops.end(), p.ops, p.ops + p.numOps);
@@ -144,7 +161,9 @@ struct DeviceBatch {
     BatchSweep *sweeps = nullptr;
     KPhase *phases = nullptr;
     KOp *ops = nullptr;
-    double2 *leanCoef = nullptr;
+    dgq::FPhase *framePhases = nullptr;
+    dgq::FOp *frameOps = nullptr;
+    double2 *frameCoef = nullptr;
     double *coef = nullptr;
     uint64_t *items = nullptr;
     uint32_t *counters = nullptr;  // ticket, then the done counters
@@ -161,7 +180,7 @@ struct DeviceBatch {
     void release() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
-        void *ptrs[] = {circ, sweeps, phases, ops, leanCoef, coef, items, counters, zsum, error};
+        void *ptrs[] = {circ, sweeps, phases, ops, framePhases, frameOps, frameCoef, coef, items, counters, zsum, error};
         for (void *p : ptrs)
             if (p) cudaFree(p);
         *this = DeviceBatch();
@@ -199,6 +218,11 @@ cudaError_t buildDevice(const std::vector<QuregState *> &regs, const std::vector
     std::vector<KPhase> phases;
     std::vector<KOp> ops;
     std::vector<double> coef;
+    std::vector<dgq::FPhase> framePhases;
+    std::vector<dgq::FOp> frameOps;
+    std::vector<double2> frameCoef;
+    const bool framed = std::all_of(plans.begin(), plans.end(), [](const RegPlan &p) { return p.framed; });
+    bool dense = false;
     d.zOff.assign(which.size(), 0);
     uint32_t doneOff = 1;  // counters[0] is the ticket
     uint32_t zOff = 0;
@@ -218,35 +242,27 @@ cudaError_t buildDevice(const std::vector<QuregState *> &regs, const std::vector
         d.zOff[i] = zOff;
         zOff += (uint32_t) s.numBits + 1;
         doneOff += c.numSweeps;
-        for (BatchSweep h : p.sweeps) {
-            h.phaseOff += (uint32_t) phases.size();
-            h.opOff += (uint32_t) ops.size();
+        for (size_t k = 0; k < p.sweeps.size(); k++) {
+            BatchSweep h = p.sweeps[k];
+            h.phaseOff = framed ? (uint32_t) framePhases.size() + p.framePhaseOff[k] : h.phaseOff + (uint32_t) phases.size();
+            h.opOff = framed ? (uint32_t) frameOps.size() + p.frameOpOff[k] : h.opOff + (uint32_t) ops.size();
             h.coefOff += (uint32_t) coef.size();
             sweeps.push_back(h);
+        }
+        if (framed) {
+            framePhases.insert(framePhases.end(), p.framePhases.begin(), p.framePhases.end());
+            frameOps.insert(frameOps.end(), p.frameOps.begin(), p.frameOps.end());
+            frameCoef.insert(frameCoef.end(), p.frameCoef.begin(), p.frameCoef.end());
+            continue;
         }
         phases.insert(phases.end(), p.phases.begin(), p.phases.end());
         ops.insert(ops.end(), p.ops.begin(), p.ops.end());
         coef.insert(coef.end(), p.coef.begin(), p.coef.end());
+        for (const KOp &op : p.ops) dense = dense || op.kind == dgq::KOP_DENSE;
     }
     d.numSweeps = (int) sweeps.size();
     d.numCounters = doneOff;
-    bool dense = false, lean = true;
-    for (const KOp &op : ops) {
-        dense = dense || op.kind == dgq::KOP_DENSE;
-        lean = lean && ((dgq::kLeanKinds >> op.kind) & 1u);
-    }
-    const int form = dense ? dgq::kBatchFormDense : lean ? dgq::kBatchFormLean : dgq::kBatchFormGeneral;
-    // the lean form reads each op's (at most two) coefficients beside its record
-    std::vector<double2> leanCoef;
-    if (form == dgq::kBatchFormLean) {
-        leanCoef.assign(ops.size(), make_double2(0.0, 0.0));
-        for (const BatchSweep &h : sweeps)
-            for (int o = 0; o < h.numOps; o++) {
-                const size_t c = (size_t) h.coefOff + ops[h.opOff + o].coef;
-                if (c < coef.size()) leanCoef[h.opOff + o].x = coef[c];
-                if (c + 1 < coef.size()) leanCoef[h.opOff + o].y = coef[c + 1];
-            }
-    }
+    const int form = framed ? dgq::kBatchFormFramed : dense ? dgq::kBatchFormDense : dgq::kBatchFormGeneral;
     d.numZ = std::max<uint32_t>(1, zOff);
 
     // work list: largest registers first; registers of several tiles in
@@ -287,7 +303,9 @@ cudaError_t buildDevice(const std::vector<QuregState *> &regs, const std::vector
     if ((e = upload(&d.sweeps, sweeps, &d.programBytes)) != cudaSuccess) return e;
     if ((e = upload(&d.phases, phases, &d.programBytes)) != cudaSuccess) return e;
     if ((e = upload(&d.ops, ops, &d.programBytes)) != cudaSuccess) return e;
-    if ((e = upload(&d.leanCoef, leanCoef, &d.programBytes)) != cudaSuccess) return e;
+    if ((e = upload(&d.framePhases, framePhases, &d.programBytes)) != cudaSuccess) return e;
+    if ((e = upload(&d.frameOps, frameOps, &d.programBytes)) != cudaSuccess) return e;
+    if ((e = upload(&d.frameCoef, frameCoef, &d.programBytes)) != cudaSuccess) return e;
     if ((e = upload(&d.coef, coef, &d.programBytes)) != cudaSuccess) return e;
     if ((e = upload(&d.items, items, &d.programBytes)) != cudaSuccess) return e;
     if ((e = cudaMalloc((void **) &d.counters, d.numCounters * sizeof(uint32_t))) != cudaSuccess) return e;
@@ -300,7 +318,9 @@ cudaError_t buildDevice(const std::vector<QuregState *> &regs, const std::vector
     a.sweeps = d.sweeps;
     a.phases = d.phases;
     a.ops = d.ops;
-    a.leanCoef = d.leanCoef;
+    a.framePhases = d.framePhases;
+    a.frameOps = d.frameOps;
+    a.frameCoef = d.frameCoef;
     a.coef = d.coef;
     a.items = d.items;
     a.numItems = (uint32_t) d.numItems;

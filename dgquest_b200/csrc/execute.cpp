@@ -379,7 +379,10 @@ int jitMinBits() {
 namespace dgq {
 
 int buildPrograms(QuregState &s, int W, std::vector<TileProgram> &out, PlanStats &st, std::string &err,
-                  bool paired, const std::function<bool(size_t)> &emit, bool folds) {
+                  bool paired, const std::function<bool(size_t)> &emit, bool interpret, bool place) {
+    const Folding folds = !interpret                            ? Folding::Specialised
+                          : place && framedGates(s.pending) ? Folding::Framed
+                                                                : Folding::None;
     // hands the programs from index `from` on to emit
     auto emitted = [&](size_t from) -> bool {
         if (!emit) return true;
@@ -413,7 +416,7 @@ int buildPrograms(QuregState &s, int W, std::vector<TileProgram> &out, PlanStats
                                                  SweepHeader hb = first ? h : SweepHeader();
                                                  const size_t from = out.size();
                                                  if (!encodeBlock(b, s.numBits, s.numQubits, W, s.pool, hb, out, &st,
-                                                                  &err, paired, folds, folds ? &carry : nullptr)) {
+                                                                  &err, paired, folds, folds != Folding::None ? &carry : nullptr)) {
                                                      code = E_UNSUPPORTED;
                                                      return false;
                                                  }
@@ -678,7 +681,9 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
         st = dgq::PlanStats();
         err.clear();
         event = 0;
-        int code = dgq::buildPrograms(s, W, s.planned, st, err, paired, emit, !interpret);
+        // (a register of one tile is over before placing diagonal gates pays:
+        // 8 us of planning for 1 us of a 10-qubit ansatz)
+        int code = dgq::buildPrograms(s, W, s.planned, st, err, paired, emit, interpret, s.numBits > W);
         if (code) return code;
         const size_t last = s.planned.size() - 1;
         for (size_t i = launched; i <= last; i++) setRenorm(s, i, last, event);

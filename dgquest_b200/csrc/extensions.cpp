@@ -3,6 +3,7 @@
 // the plan/launch split, cost-model settings, device state access, the
 // host-only planner and kernel-source calls, the FP64 peak probe.
 #include "api_internal.h"
+#include "frame.h"
 
 using dgq::Gate;
 
@@ -502,6 +503,41 @@ int dgq_sweepSourceKey(int numQubits, int tileBits, int count, const int32_t *ty
     std::strncpy(buf, src.c_str(), (size_t) len - 1);
     buf[len - 1] = '\0';
     return (int) src.size() < len ? (int) s.planned.size() : -2;
+}
+
+int dgq_frameApplyHost(int numQubits, int tileBits, int count, const int32_t *types, const uint64_t *targetMasks,
+                       const uint64_t *controlMasks, const double *operands, double *re, double *im) {
+    if (numQubits < dgq::kMinTileBits || numQubits > 16 || tileBits < dgq::kMinTileBits || tileBits > numQubits ||
+        tileBits > dgq::kMaxTileBitsF64 || count < 0 || !re || !im ||
+        (count > 0 && (!types || !targetMasks || !controlMasks || !operands))) {
+        raise(E_INVALID_ARGUMENT, __func__);
+        return -1;
+    }
+    QuregState s;
+    s.numQubits = s.numBits = numQubits;
+    resetMapping(s);
+    if (!gatesFromArrays(numQubits, count, types, targetMasks, controlMasks, operands, s.pending, __func__)) return -1;
+    dgq::PlanStats st;
+    std::string err;
+    if (int code = dgq::buildPrograms(s, tileBits, s.planned, st, err)) {
+        raise(code, __func__, err.c_str());
+        return -1;
+    }
+    std::vector<dgq::FrameSweep> sweeps(s.planned.size());
+    for (size_t i = 0; i < sweeps.size(); i++)
+        if (!dgq::frameProgram(s.planned[i], tileBits, sweeps[i])) return 0;
+    const size_t D = (size_t) 1 << numQubits;
+    std::vector<double> v(2 * D);
+    for (size_t i = 0; i < D; i++) {
+        v[2 * i] = re[i];
+        v[2 * i + 1] = im[i];
+    }
+    for (size_t i = 0; i < sweeps.size(); i++) dgq::applyFramedHost(s.planned[i], sweeps[i], tileBits, v.data());
+    for (size_t i = 0; i < D; i++) {
+        re[i] = v[2 * i];
+        im[i] = v[2 * i + 1];
+    }
+    return (int) sweeps.size();
 }
 
 int dgq_specialiseGates(int numQubits, int precision, int count, const int32_t *types, const uint64_t *targetMasks,

@@ -1,7 +1,8 @@
 // kernels.cu -- the sm_100a kernels of the FP64 state-vector path.
 //
-//   tileKernel<W,V,LEAN> one sweep of the state applying a fused block
+//   frameKernel<W,V> one sweep of the state applying a fused block
 //                    (dgQuEST statevec_fusedKernel, QuEST_gpu_kernel.cu:175-359)
+//   tileKernel<W,V>  the same for programs without a framed form
 //   probKernel       P(bit = 0) for every address bit in one read pass
 //   probFinalize     (statevec_findProbabilityOfZeroKernel + reducePingpong,
 //                    QuEST_gpu_kernel.cu:656-840)
@@ -15,7 +16,9 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 
+#include "frame.cuh"
 #include "interp.cuh"
 #include "kernels.h"
 #include "tile_program.h"
@@ -24,36 +27,30 @@ namespace dgq {
 
 __device__ __forceinline__ uint32_t swz(uint32_t x) { return x ^ (((x >> 3) ^ (x >> 6) ^ (x >> 9) ^ (x >> 12)) & 7u); }
 
-// ------------------------------------------------------------ tile kernel
-// 128 registers per thread: 16 warps per SM at every tile width. V is
-// double2 (complex128) or float2 (complex64, with the per-sweep
-// renormalisation of the complex64 form: scale by 1/sqrt(*normIn) with the
-// global factor, add the output's sum of |a|^2 to *normOut).
-template <int W, class V, bool LEAN>
-__global__ void __launch_bounds__(1 << (W - kRegBits), 65536 / (128 << (W - kRegBits)))
-    tileKernel(V *__restrict__ st, const __grid_constant__ TileProgram prog) {
-    typedef typename Real<V>::T R;
-    constexpr int T = 1 << (W - kRegBits);
-    extern __shared__ __align__(16) unsigned char smRaw[];
-    V *sm = reinterpret_cast<V *>(smRaw);
-    const uint32_t tid = threadIdx.x;
-    const uint32_t cta = blockIdx.x + prog.ctaOffset;
-
-    // address of canonical element (tid, j): base | lane bits | thread high bits | j bits
-    uint64_t tpart = tid & 31u;
-    const int nCta = prog.numBits - W;
-    for (int i = 0; i < nCta; i++) tpart |= (uint64_t) ((cta >> i) & 1u) << prog.ctaPos[i];
+// ------------------------------------------------------------ tile kernels
+// Canonical order of a tile: element (tid, j) at base | lane bits | thread
+// high bits | j bits. Prog: TileProgram or FrameProgram.
+template <int W>
+struct TileAddress {
+    uint64_t tpart, jb[kRegBits];
+    template <class Prog>
+    __device__ __forceinline__ TileAddress(const Prog &prog, uint32_t tid, uint32_t cta) {
+        tpart = tid & 31u;
+        const int nCta = prog.numBits - W;
+        for (int i = 0; i < nCta; i++) tpart |= (uint64_t) ((cta >> i) & 1u) << prog.ctaPos[i];
 #pragma unroll
-    for (int i = 0; i < W - 9; i++) tpart |= (uint64_t) ((tid >> (5 + i)) & 1u) << prog.highPos[i];
-    const uint64_t jb0 = 1ULL << prog.highPos[W - 9];
-    const uint64_t jb1 = 1ULL << prog.highPos[W - 8];
-    const uint64_t jb2 = 1ULL << prog.highPos[W - 7];
-    const uint64_t jb3 = 1ULL << prog.highPos[W - 6];
-    auto gidx = [&](int j) -> uint64_t {
-        return tpart | ((j & 1) ? jb0 : 0ULL) | ((j & 2) ? jb1 : 0ULL) | ((j & 4) ? jb2 : 0ULL) | ((j & 8) ? jb3 : 0ULL);
-    };
+        for (int i = 0; i < W - 9; i++) tpart |= (uint64_t) ((tid >> (5 + i)) & 1u) << prog.highPos[i];
+#pragma unroll
+        for (int b = 0; b < kRegBits; b++) jb[b] = 1ULL << prog.highPos[W - 9 + b];
+    }
+    __device__ __forceinline__ uint64_t operator()(int j) const {
+        return tpart | ((j & 1) ? jb[0] : 0ULL) | ((j & 2) ? jb[1] : 0ULL) | ((j & 4) ? jb[2] : 0ULL) | ((j & 8) ? jb[3] : 0ULL);
+    }
+};
 
-    V a[kRegs];
+template <int W, class V, class Prog>
+__device__ __forceinline__ void loadTile(const V *st, const Prog &prog, const TileAddress<W> &gidx, V (&a)[kRegs]) {
+    typedef typename Real<V>::T R;
     if (prog.initKind == INIT_NONE) {
 #pragma unroll
         for (int j = 0; j < kRegs; j++) a[j] = st[gidx(j)];
@@ -82,6 +79,43 @@ __global__ void __launch_bounds__(1 << (W - kRegBits), 65536 / (128 << (W - kReg
             a[j] = keep ? mk<V>(a[j].x * sc, a[j].y * sc) : mk<V>((R) 0, (R) 0);
         }
     }
+}
+
+// Adds the tile's sum of |a|^2 to *normOut.
+template <int T, class V>
+__device__ __forceinline__ void addNorm(const V (&a)[kRegs], uint32_t tid, double *normOut) {
+    __shared__ double red[32];
+    double acc = 0.0;
+#pragma unroll
+    for (int j = 0; j < kRegs; j++) acc += (double) a[j].x * (double) a[j].x + (double) a[j].y * (double) a[j].y;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if ((tid & 31u) == 0) red[tid >> 5] = acc;
+    __syncthreads();
+    if (tid == 0) {
+        double t = 0.0;
+        for (int w = 0; w < T / 32; w++) t += red[w];
+        atomicAdd(normOut, t);
+    }
+}
+
+// 128 registers per thread: 16 warps per SM at every tile width. V is
+// double2 (complex128) or float2 (complex64, with the per-sweep
+// renormalisation of the complex64 form: scale by 1/sqrt(*normIn) with the
+// global factor, add the output's sum of |a|^2 to *normOut).
+// Programs with an op that no framed program holds (frame.h).
+template <int W, class V>
+__global__ void __launch_bounds__(1 << (W - kRegBits), 65536 / (128 << (W - kRegBits)))
+    tileKernel(V *__restrict__ st, const __grid_constant__ TileProgram prog) {
+    typedef typename Real<V>::T R;
+    constexpr int T = 1 << (W - kRegBits);
+    extern __shared__ __align__(16) unsigned char smRaw[];
+    V *sm = reinterpret_cast<V *>(smRaw);
+    const uint32_t tid = threadIdx.x;
+    const uint32_t cta = blockIdx.x + prog.ctaOffset;
+    const TileAddress<W> gidx(prog, tid, cta);
+    V a[kRegs];
+    loadTile<W>(st, prog, gidx, a);
 
     const int numPhases = prog.numPhases;
     if (numPhases > 0) {
@@ -97,7 +131,7 @@ __global__ void __launch_bounds__(1 << (W - kRegBits), 65536 / (128 << (W - kReg
 #pragma unroll
             for (int j = 0; j < kRegs; j++) a[j] = sm[sb ^ ph.regOff[j]];
             const int e = ph.opEnd;
-            for (int o = ph.opBegin; o < e; o++) applyOp<V, !LEAN, LEAN>(prog.ops[o], prog.coef, a, loc, cta);
+            for (int o = ph.opBegin; o < e; o++) applyOp<V, true>(prog.ops[o], prog.coef, a, loc, cta);
 #pragma unroll
             for (int j = 0; j < kRegs; j++) sm[sb ^ ph.regOff[j]] = a[j];
             __syncthreads();
@@ -116,43 +150,79 @@ __global__ void __launch_bounds__(1 << (W - kRegBits), 65536 / (128 << (W - kReg
 #pragma unroll
         for (int j = 0; j < kRegs; j++) a[j] = mk<V>(gr * a[j].x - gi * a[j].y, gr * a[j].y + gi * a[j].x);
     }
-    if (prog.renormOut) {
-        __shared__ double red[32];
-        double acc = 0.0;
-#pragma unroll
-        for (int j = 0; j < kRegs; j++) acc += (double) a[j].x * (double) a[j].x + (double) a[j].y * (double) a[j].y;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if ((tid & 31u) == 0) red[tid >> 5] = acc;
-        __syncthreads();
-        if (tid == 0) {
-            double t = 0.0;
-            for (int w = 0; w < T / 32; w++) t += red[w];
-            atomicAdd(prog.normOut, t);
-        }
-    }
+    if (prog.renormOut) addNorm<T>(a, tid, prog.normOut);
 #pragma unroll
     for (int j = 0; j < kRegs; j++) st[gidx(j)] = a[j];
 }
 
-template <int W, class V, bool LEAN>
-static cudaError_t launchTileWL(V *st, const TileProgram &prog, cudaStream_t s) {
-    static std::atomic<uint64_t> optIn{0};
-    const size_t smem = sizeof(V) << W;
-    cudaError_t e = ensureSmemOptIn((const void *) tileKernel<W, V, LEAN>, (int) smem, optIn);
-    if (e != cudaSuccess) return e;
-    const unsigned grid = prog.ctaCount ? prog.ctaCount : 1u << (prog.numBits - W);
-    tileKernel<W, V, LEAN><<<grid, 1 << (W - kRegBits), smem, s>>>(st, prog);
-    return cudaGetLastError();
+// The framed form (frame.h).
+template <int W, class V>
+__global__ void __launch_bounds__(1 << (W - kRegBits), 65536 / (128 << (W - kRegBits)))
+    frameKernel(V *__restrict__ st, const __grid_constant__ FrameProgram prog) {
+    constexpr int T = 1 << (W - kRegBits);
+    extern __shared__ __align__(16) unsigned char smRaw[];
+    V *sm = reinterpret_cast<V *>(smRaw);
+    const uint32_t tid = threadIdx.x;
+    const uint32_t cta = blockIdx.x + prog.ctaOffset;
+    V a[kRegs];
+    loadTile<W>(st, prog, TileAddress<W>(prog, tid, cta), a);
+    if (prog.numPhases > 0) {
+#pragma unroll
+        for (int j = 0; j < kRegs; j++) sm[swz(tid + (uint32_t) (T * j))] = a[j];
+        __syncthreads();
+        framePhases<V, W>(
+            prog.numPhases, prog.tail, sm, tid, cta, [&](int p) -> const FPhase & { return prog.phases[p]; },
+            [&](int o) -> const FOp & { return prog.ops[o]; },
+            [&](int o) { return make_double2(prog.coef[2 * o], prog.coef[2 * o + 1]); }, [] { __syncthreads(); });
+#pragma unroll
+        for (int j = 0; j < kRegs; j++) a[j] = sm[swz(tid + (uint32_t) (T * j))];
+    }
+    frameFinish(prog.tail, a, tid, cta, prog.renormIn != 0, prog.renormIn ? rsqrt(*prog.normIn) : 1.0);
+    if (prog.renormOut) addNorm<T>(a, tid, prog.normOut);
+    const TileAddress<W> gidx(prog, tid, cta);
+#pragma unroll
+    for (int j = 0; j < kRegs; j++) st[gidx(j)] = a[j];
 }
 
-// The lean form when every op of the program is a lean kind (rotations,
-// CNOT, CZ, phases): measured 10-11 % faster on a 28-qubit random circuit.
 template <int W, class V>
 static cudaError_t launchTileW(V *st, const TileProgram &prog, cudaStream_t s) {
-    bool lean = true;
-    for (int i = 0; i < prog.numOps && lean; i++) lean = (kLeanKinds >> prog.ops[i].kind) & 1u;
-    return lean ? launchTileWL<W, V, true>(st, prog, s) : launchTileWL<W, V, false>(st, prog, s);
+    const size_t smem = sizeof(V) << W;
+    const unsigned grid = prog.ctaCount ? prog.ctaCount : 1u << (prog.numBits - W);
+    FrameSweep f;
+    if (!frameProgram(prog, W, f)) {
+        static std::atomic<uint64_t> optIn{0};
+        cudaError_t e = ensureSmemOptIn((const void *) tileKernel<W, V>, (int) smem, optIn);
+        if (e != cudaSuccess) return e;
+        tileKernel<W, V><<<grid, 1 << (W - kRegBits), smem, s>>>(st, prog);
+        return cudaGetLastError();
+    }
+    static std::atomic<uint64_t> optIn{0};
+    cudaError_t e = ensureSmemOptIn((const void *) frameKernel<W, V>, (int) smem, optIn);
+    if (e != cudaSuccess) return e;
+    FrameProgram fp;
+    fp.numPhases = prog.numPhases;
+    fp.numBits = prog.numBits;
+    fp.numReal = prog.numReal;
+    fp.initKind = prog.initKind;
+    fp.hasRestrict = prog.hasRestrict;
+    fp.renormIn = prog.renormIn;
+    fp.renormOut = prog.renormOut;
+    fp.normIn = prog.normIn;
+    fp.normOut = prog.normOut;
+    fp.initIndex = prog.initIndex;
+    fp.initAmp = prog.initAmp;
+    fp.restrictMask = prog.restrictMask;
+    fp.restrictValue = prog.restrictValue;
+    fp.restrictScale = prog.restrictScale;
+    fp.ctaOffset = prog.ctaOffset;
+    std::memcpy(fp.highPos, prog.highPos, sizeof(fp.highPos));
+    std::memcpy(fp.ctaPos, prog.ctaPos, sizeof(fp.ctaPos));
+    fp.tail = f.tail;
+    std::copy(f.phases.begin(), f.phases.end(), fp.phases);
+    std::copy(f.ops.begin(), f.ops.end(), fp.ops);
+    std::copy(f.coef.begin(), f.coef.end(), fp.coef);
+    frameKernel<W, V><<<grid, 1 << (W - kRegBits), smem, s>>>(st, fp);
+    return cudaGetLastError();
 }
 
 template <class V>

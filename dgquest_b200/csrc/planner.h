@@ -71,16 +71,25 @@ struct SweepHeader {
     double restrictScale = 1.0;
 };
 
+// The kernel a program is for, as far as the plan depends on it.
+enum class Folding { None, Framed, Specialised };
+
 // paired: encode for the complex64 paired form (TileProgram::paired); fails
 // (with *err set) on a multi-qubit unitary that targets address bit 0.
-// folds: the program is for a specialised kernel, which folds phase factors
-// on thread bits into one factor per thread; diagonal gates then move to the
-// phases where they are such factors. carry (with folds): diagonal gates of
+// folds: the program is for a kernel that folds phase factors on thread bits
+// into one factor per thread (a specialised one, or the framed interpreter);
+// diagonal gates then move to the phases where they are such factors. carry (with folds): diagonal gates of
 // the block before, run first here; the block's own that would be cheaper in
 // the next block are left in it (none when the block is the last).
 bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits, const MatrixPool &pool,
                  const SweepHeader &first, std::vector<TileProgram> &out, PlanStats *stats, std::string *err,
-                 bool paired = false, bool folds = false, std::vector<Gate> *carry = nullptr);
+                 bool paired = false, Folding folds = Folding::None, std::vector<Gate> *carry = nullptr);
+
+// Whether the framed interpreter is likely to run every gate (frame.h; a
+// general 2x2 without controls may still turn out to have no framed form,
+// and then runs on the other interpreter, which runs any plan but the
+// specialised kernels').
+bool framedGates(const std::vector<Gate> &gates);
 
 // A program that only applies the header (init and/or lazy collapse).
 void encodeHeaderOnly(int numBits, int numReal, int tileBits, const SweepHeader &hdr, TileProgram &out,

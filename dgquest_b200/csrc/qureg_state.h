@@ -120,11 +120,14 @@ namespace dgq {
 // error code with err set. The register is not changed.
 // paired: the complex64 paired form (TileProgram::paired; W counts the
 // in-slot bit, so W - 1 tile bits index 16-byte slots).
+// interpret: for the interpreting kernels, else for specialised ones; place:
+// move diagonal gates to their cheapest phase there too.
 // emit (if set) is called with the index of each program as soon as it is
 // complete, in order; when it returns false, planning stops and
 // buildPrograms returns -1 (the callback has reported its own error).
 int buildPrograms(QuregState &s, int W, std::vector<TileProgram> &out, PlanStats &st, std::string &err,
-                  bool paired = false, const std::function<bool(size_t)> &emit = nullptr, bool folds = false);
+                  bool paired = false, const std::function<bool(size_t)> &emit = nullptr, bool interpret = true,
+                  bool place = true);
 // Drops the pending work that buildPrograms planned (after it has been
 // launched or kept for launching).
 void consumePending(QuregState &s);

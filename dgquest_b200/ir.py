@@ -83,6 +83,26 @@ def fuse_apply_host(n, k, types, tm, cm, opnd, amps):
     return re + 1j * im, nb
 
 
+def frame_apply_host(n, tile_bits, types, tm, cm, opnd, amps):
+    """The framed sweep programs on the host: gates (IR arrays) planned with
+    tiles of 2^tile_bits amplitudes and applied in FP64 to amps (length 2^n);
+    returns (new amps, number of sweeps), 0 sweeps when one has no framed form."""
+    from .quest import _check, _library
+    P = ctypes.POINTER
+    re = np.ascontiguousarray(amps.real, dtype=np.float64).copy()
+    im = np.ascontiguousarray(amps.imag, dtype=np.float64).copy()
+    t = np.ascontiguousarray(types, dtype=np.int32)
+    tm = np.ascontiguousarray(tm, dtype=np.uint64)
+    cm = np.ascontiguousarray(cm, dtype=np.uint64)
+    o = np.ascontiguousarray(opnd, dtype=np.float64).reshape(-1, 8)
+    sweeps = _library().dgq_frameApplyHost(n, tile_bits, len(t), t.ctypes.data_as(P(ctypes.c_int32)),
+                                           tm.ctypes.data_as(P(ctypes.c_uint64)), cm.ctypes.data_as(P(ctypes.c_uint64)),
+                                           o.ctypes.data_as(P(ctypes.c_double)), re.ctypes.data_as(P(ctypes.c_double)),
+                                           im.ctypes.data_as(P(ctypes.c_double)))
+    _check()
+    return re + 1j * im, sweeps
+
+
 def plan_exchanges(ops, n, local_qubits, batch):
     """Host-only: (segments, exchange passes, qubits moved) of an op list on
     a register whose pages (batch=False, host tier) or shards (batch=True)

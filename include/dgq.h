@@ -235,6 +235,14 @@ int dgq_planExchanges(int numQubits, int localQubits, int batch, int count, cons
 int dgq_fuseApplyHost(int numQubits, int K, int count, const int32_t *types, const uint64_t *targetMasks,
                       const uint64_t *controlMasks, const double *operands, double *re, double *im);
 
+/* Host only (no GPU): plans the gates (dgq_planGates encoding, checked the
+ * same way) for the interpreting kernels with tiles of 2^tileBits amplitudes
+ * and applies the framed sweep programs to 2^numQubits amplitudes (9..16
+ * qubits). Returns the number of sweeps, or 0 with the amplitudes unchanged
+ * when a sweep has no framed form. */
+int dgq_frameApplyHost(int numQubits, int tileBits, int count, const int32_t *types, const uint64_t *targetMasks,
+                       const uint64_t *controlMasks, const double *operands, double *re, double *im);
+
 /* Registers with at least minBits address bits run runtime-specialised
  * sweep kernels (default 22, or DGQ_JIT_MIN_BITS; DGQ_JIT=0 disables
  * specialisation). Negative restores the default. Returns the previous value. */

@@ -1,0 +1,81 @@
+"""Framed sweep programs on the GPU (csrc/frame.h, the interpreting kernels):
+every framed gate kind at every tile width in both precisions, with CNOT, CZ
+and Pauli gates between rotations on tile, thread and CTA bits, a collapse
+between two parts, and batches that are framed or not, against the oracle.
+
+Bound: the same factors as the gate-by-gate product, so 1e-12 per amplitude
+in complex128 and fidelity 1 - 1e-6 in complex64."""
+import numpy as np
+import pytest
+
+import oracle
+from dgquest_b200 import circuits as C
+
+pytestmark = pytest.mark.gpu
+
+FRAMED = [C.H, C.X, C.Y, C.Z, C.S, C.T, C.RX, C.RY, C.RZ, C.PHASE, C.CNOT, C.CNOT, C.CZ, C.CPHASE, C.CRZ, C.SQX, C.SQY,
+          C.SQW, C.COMPACT, C.UNITARY, C.SWAP]
+
+
+def check(amps, ref, single):
+    if single:
+        assert abs(np.vdot(ref, amps)) ** 2 / np.vdot(amps, amps).real >= 1 - 1e-6
+    else:
+        assert np.abs(amps - ref).max() <= 1e-12
+
+
+@pytest.mark.parametrize("single", [False, True])
+@pytest.mark.parametrize("n,width", [(2, 9), (5, 9), (9, 9), (10, 9), (13, 9), (12, 10), (13, 11), (12, 12), (15, 12)])
+def test_framed_sweeps_match_oracle(quest, env, n, width, single):
+    Q = quest
+    ops = np.concatenate([C.mixed_ops(n, 250, 31 * n + width, kinds=FRAMED), C.hea(n, 4, n)])
+    q = Q.dgq_createQuregF32(n, env) if single else Q.createQureg(n, env)
+    try:
+        Q.dgq_setTileBits(q, width)
+        Q.dgq_setDenseFusion(q, 0)
+        C.replay(q, ops)
+        amps = Q.state_vector(q)
+    finally:
+        Q.destroyQureg(q, env)
+    check(amps, oracle.run(n, ops)[0], single)
+
+
+def test_collapse_between_framed_sweeps(quest, env):
+    Q, n = quest, 14
+    b = C.OpList()
+    for t in (3, 12):
+        b.add(C.MEASURE, t)
+    ops = np.concatenate([C.mixed_ops(n, 150, 5, kinds=FRAMED), b.array(), C.mixed_ops(n, 150, 6, kinds=FRAMED)])
+    q = Q.createQureg(n, env)
+    try:
+        Q.seed([77])
+        outcomes = C.replay(q, ops)
+        amps = Q.state_vector(q)
+    finally:
+        Q.destroyQureg(q, env)
+    ref = oracle.run(n, ops, seed_keys=[77])
+    assert list(outcomes) == list(ref[2])
+    check(amps, ref[0], False)
+
+
+@pytest.mark.parametrize("unframed", [False, True])
+def test_batches_with_and_without_a_framed_form(quest, env, unframed):
+    Q = quest
+    sizes = [9, 10, 12, 13, 14]
+    lists = [C.mixed_ops(n, 200, 40 + n, kinds=FRAMED) for n in sizes]
+    if unframed:
+        lists[2] = np.concatenate([lists[2], C.mixed_ops(sizes[2], 5, 9, kinds=[C.CRX])])
+    regs = [Q.createQureg(n, env) for n in sizes]
+    try:
+        for q, ops in zip(regs, lists):
+            C.replay(q, ops)
+        b = Q.Batch(regs, config={"tileBits": 12})
+        b.launch()
+        b.wait()
+        states = [Q.state_vector(q) for q in regs]
+        b.close()
+    finally:
+        for q in regs:
+            Q.destroyQureg(q, env)
+    for n, ops, a in zip(sizes, lists, states):
+        check(a, oracle.run(n, ops)[0], False)
