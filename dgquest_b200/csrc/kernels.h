@@ -49,6 +49,16 @@ struct SwapArgs {
     uint8_t b[32];
 };
 
+// The exchange as a permutation of tiles: tile-local bit i is address bit
+// tilePos[i]; tiles are numbered by the other bits (outPos). Both sets are
+// closed under the exchange.
+struct SwapTileArgs {
+    int32_t tileBits, outBits;
+    int32_t tilePairs, outPairs;     // pairs of tile-local bits, of address bits outside the tile
+    uint8_t tileA[16], tileB[16], outA[32], outB[32];
+    uint8_t tilePos[16], outPos[kMaxStateBits];
+};
+
 struct GatherArgs {
     uint64_t begin, count;
     uint64_t stride;  // logical index of entry i: begin + i * stride (0 means 1)
