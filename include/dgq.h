@@ -345,7 +345,7 @@ int64_t dgq_getAvailableMemory(void);
 typedef struct dgq_batch_s *dgq_batch;
 typedef struct dgq_batch_config {
     int32_t tileBits;     /* widest tile, 9..12 (registers narrower than it use their width); 0 = choose */
-    int32_t groupFactor;  /* registers interleaved sweep by sweep: about groupFactor x grid tiles; 0 = choose */
+    int32_t groupFactor;  /* registers worked on at a time: those of at most groupFactor x grid tiles; 0 = choose */
     int32_t ctasPerSm;    /* persistent CTAs per SM; 0 = as many as fit */
     int32_t tune;         /* 1: time candidate tile widths and group factors on a sample of the batch */
 } dgq_batch_config;
