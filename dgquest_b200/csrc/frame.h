@@ -17,6 +17,13 @@
 // to which the phase writes its result, S by the last pass of the sweep.
 // Phases on thread and CTA bits alone are one number per thread: they come
 // first in a phase, in a loop that touches no amplitude.
+//
+// Bound: latency and instruction issue of the dispatch, with 16 warps an SM
+// at 128 registers (issue 40 % of the cycles, FP64 pipe 19..28 %, DRAM idle);
+// a register of one tile waits mostly for instruction fetches. Measured
+// against the form with CNOT operations: a batch of 48 registers of 10..20
+// qubits 5.30 -> 4.25 ms, the five sweeps of a 21-qubit Fourier transform
+// 248 -> 190 us, one tile of a 10-qubit ansatz 33.9 -> 26.8 us.
 #pragma once
 
 #include <cstdint>
