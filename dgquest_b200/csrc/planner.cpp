@@ -591,24 +591,6 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
     };
     TileProgram *prog = newProgram(true);
     int numCoef = 0;
-    // The interpreting kernels' global factor is multiplied up in extended
-    // precision and rounded once per phase: an error in it is the same for
-    // every amplitude (12 qubits, 20 random layers: 1.4e-15 -> 1.0e-15 of the
-    // state's norm).
-    const bool extended = folds != Folding::Specialised;
-    long double globalRe = 1.0L, globalIm = 0.0L;
-    auto multiply = [&](long double &re, long double &im, long double fr, long double fi) {
-        if (extended) {
-            const long double r = re * fr - im * fi, i = re * fi + im * fr;
-            re = r;
-            im = i;
-        } else {
-            const double a = (double) re, b = (double) im, c = (double) fr, d = (double) fi;
-            const double r = a * c - b * d, i = a * d + b * c;
-            re = r;
-            im = i;
-        }
-    };
 
     for (const Phase &ph : phases) {
         const PhaseLayout L = makeLayout(ph.front, ph.targetsLocal, tileBits, paired);
@@ -616,8 +598,12 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
         // rotations leave their scalar factor in (phRe, phIm)
         std::vector<KOp> ops;
         std::vector<double> coef;
-        long double phRe = 1.0L, phIm = 0.0L;
-        auto scaleBy = [&](long double fr, long double fi) { multiply(phRe, phIm, fr, fi); };
+        double phRe = 1.0, phIm = 0.0;
+        auto scaleBy = [&](double fr, double fi) {
+            const double r = phRe * fr - phIm * fi, i = phRe * fi + phIm * fr;
+            phRe = r;
+            phIm = i;
+        };
         for (const Gate &g : ph.gates) {
             KOp op;
             std::memset(&op, 0, sizeof(op));
@@ -717,7 +703,7 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
                             coef.insert(coef.end(), {kRsqrt2, kRsqrt2, kRsqrt2, -kRsqrt2});
                         } else {
                             op.kind = KOP_H1;
-                            scaleBy(extended ? 0.707106781186547524400844362104849L : kRsqrt2, 0.0);
+                            scaleBy(kRsqrt2, 0.0);
                         }
                         break;
                     case OP_ROTATE_Y:
@@ -828,13 +814,11 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
             numCoef + (int) coef.size() > kMaxCoef) {
             prog = newProgram(false);
             numCoef = 0;
-            globalRe = 1.0L;
-            globalIm = 0.0L;
         }
-        if (phRe != 1.0L || phIm != 0.0L) {
-            multiply(globalRe, globalIm, phRe, phIm);
-            prog->globalRe = (double) globalRe;
-            prog->globalIm = (double) globalIm;
+        if (phRe != 1.0 || phIm != 0.0) {
+            const double gr = prog->globalRe, gi = prog->globalIm;
+            prog->globalRe = gr * phRe - gi * phIm;
+            prog->globalIm = gr * phIm + gi * phRe;
             prog->hasGlobal = 1;
         }
         KPhase &kp = prog->phases[prog->numPhases++];
