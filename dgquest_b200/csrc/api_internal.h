@@ -139,7 +139,7 @@ void readCostFileExtras(const char *path, CostModel &cm);
 bool readCostFile(const char *path, double &sweepMs, double &phaseMs);
 CostModel costModel();
 double predictPlanSeconds(const std::vector<Gate> &gates, int numBits, int W, const dgq::MatrixPool &pool,
-                          int lookahead);
+                          int lookahead, bool paired = false);
 int chooseTileBits(QuregState &s);
 double predictDenseSeconds(const QuregState &s, int K, int *blocksOut, double bound, bool *stopped);
 int chooseForm(QuregState &s);

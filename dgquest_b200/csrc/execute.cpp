@@ -110,7 +110,7 @@ bool isWide(const Gate &g) { return g.type == dgq::OP_MULTI_UNITARY && g.numMult
 // four 6-qubit unitaries, 7 extra dense sweeps of 0.81 ms for 3 tile sweeps
 // of 0.34 ms.)
 double predictPlanSeconds(const std::vector<Gate> &gates, int numBits, int W, const dgq::MatrixPool &pool,
-                          int lookahead) {
+                          int lookahead, bool paired) {
     const CostModel cm = costModel();
     const double amps = std::ldexp(1.0, numBits);
     std::vector<dgq::TileProgram> progs;
@@ -118,9 +118,10 @@ double predictPlanSeconds(const std::vector<Gate> &gates, int numBits, int W, co
     dgq::SweepHeader h;
     std::string err;
     auto count = [&](const std::vector<Gate> &seg) {
-        for (const auto &b : dgq::planBlocks(seg, numBits, W, nullptr, dgq::kCoalescedBits, lookahead)) {
+        const int seed = dgq::kCoalescedBits + (paired ? 1 : 0);
+        for (const auto &b : dgq::planBlocks(seg, numBits, W, nullptr, seed, lookahead)) {
             progs.clear();
-            if (!dgq::encodeBlock(b, numBits, numBits, W, pool, h, progs, &st, &err)) return false;
+            if (!dgq::encodeBlock(b, numBits, numBits, W, pool, h, progs, &st, &err, paired)) return false;
         }
         return true;
     };
@@ -180,6 +181,10 @@ int chooseTileBits(QuregState &s) {
     for (int W = lo; W <= hi; W++) {
         if (dgq::lookaheadBySize(s.numBits)) cands.push_back({W, 1, 1e300});
         cands.push_back({W, 0, 1e300});
+        if (W == hi && dgq::lookaheadBySize(s.numBits)) {
+            cands.push_back({W, dgq::kSearchBeam4, 1e300});
+            cands.push_back({W, dgq::kSearchBeam16, 1e300});
+        }
     }
     {
         std::vector<std::thread> th;
@@ -203,6 +208,24 @@ int chooseTileBits(QuregState &s) {
     }
     s.predictedTileSeconds = bestT;
     return best;
+}
+
+int pairedTileBits(const QuregState &s);
+
+// The paired form's block search (its width is given): the predicted best.
+int choosePairedSearch(const QuregState &s, int W) {
+    if (!dgq::lookaheadBySize(s.numBits)) return -1;
+    const int search[3] = {1, dgq::kSearchBeam4, dgq::kSearchBeam16};
+    double t[3];
+    auto plan = [&](int i) { t[i] = predictPlanSeconds(s.pending, s.numBits, W, s.pool, search[i], true); };
+    std::thread a(plan, 1), b(plan, 2);
+    plan(0);
+    a.join();
+    b.join();
+    int best = 0;
+    for (int i = 1; i < 3; i++)
+        if (t[i] < t[best]) best = i;
+    return search[best];
 }
 
 // Predicted time of the dense-block form with K-qubit blocks: the blocks'
@@ -243,7 +266,7 @@ double predictDenseSeconds(const QuregState &s, int K, int *blocksOut, double bo
 // less than optimal, never wrong). It saves the candidate planning, about
 // 6 ms of a 30-qubit circuit's 10 ms of planning.
 struct FormChoice {
-    int formK = 0, tileBits = 0, lookahead = -1;
+    int formK = 0, tileBits = 0, lookahead = -1, pairedLookahead = -1;
     double tileSeconds = 0.0;
     dgq_plan_stats stats{};
 };
@@ -285,6 +308,7 @@ int chooseForm(QuregState &s) {
             const FormChoice &f = it->second;
             s.formTileBits = f.tileBits;
             s.formLookahead = f.lookahead;
+            s.formPairedLookahead = f.pairedLookahead;
             s.planLookahead = f.lookahead;
             s.predictedTileSeconds = f.tileSeconds;
             s.stats.predictedTileMs = f.stats.predictedTileMs;
@@ -298,6 +322,7 @@ int chooseForm(QuregState &s) {
     f.formK = formK;
     f.tileBits = s.formTileBits;
     f.lookahead = s.formLookahead;
+    f.pairedLookahead = s.formPairedLookahead;
     f.tileSeconds = s.predictedTileSeconds;
     f.stats = s.stats;
     std::lock_guard<std::mutex> lk(g_formMutex);
@@ -311,6 +336,7 @@ int chooseFormUncached(QuregState &s, const CostModel &cm) {
     // block counting stops as soon as they cannot win
     s.formTileBits = chooseTileBits(s);
     s.formLookahead = s.planLookahead;
+    s.formPairedLookahead = s.single ? choosePairedSearch(s, pairedTileBits(s)) : -1;
     double tile = s.predictedTileSeconds;
     if (s.single) tile *= cm.c64TileFactor;
     tile += wideSeconds(s, s.pending, dgq::kRegBits, cm);
@@ -593,6 +619,7 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
     const double t0 = nowMillis();
     int denseBlocks = 0;
     int formK = s.denseFusion > 0 ? s.denseFusion : 0;
+    s.formPairedLookahead = -1;
     s.stats.formAuto = 0;
     s.formTileBits = 0;
     s.stats.predictedTileMs = 0.0;
@@ -670,6 +697,7 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
         s.planLookahead = -1;
         if (paired) {
             W = pairedTileBits(s);
+            if (formK == 0) s.planLookahead = s.formPairedLookahead;
         } else if (s.formTileBits > 0 && formK == 0) {
             // the form choice planned the tile widths already
             W = s.formTileBits;

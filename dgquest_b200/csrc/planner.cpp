@@ -90,6 +90,38 @@ static void growMask(const GateDag &dag, u64 &mask, int budget, bool preferHigh,
     }
 }
 
+// Grows `mask` keeping the `width` masks of each size that let the most gates
+// run, and takes the best of all. Greedy growth commits to every bit: on 30
+// qubits at depth 20 a width of 16 saves 0..2 of 18 sweeps, 4 saves 4 of 17
+// on a 26-qubit ansatz of depth 10, and on a 4 x 7 grid greedy growth is the
+// better one (12 sweeps, 13), so the cost model plans with each.
+static void beamMask(const GateDag &dag, u64 &mask, int budget, size_t width) {
+    std::vector<u64> beam{mask}, sets, next;
+    std::vector<size_t> counts, rank;
+    size_t bestCount = 0;
+    while (!beam.empty()) {
+        sets.clear();
+        for (u64 m : beam)
+            for (u64 add : dag.frontierSets(m))
+                if (popcount64(m | add) <= budget && std::find(sets.begin(), sets.end(), m | add) == sets.end())
+                    sets.push_back(m | add);
+        counts.resize(sets.size());
+        rank.resize(sets.size());
+        dag.countAllowed(sets.data(), sets.size(), counts.data());
+        for (size_t i = 0; i < sets.size(); i++) {
+            rank[i] = i;
+            if (counts[i] > bestCount) {
+                bestCount = counts[i];
+                mask = sets[i];
+            }
+        }
+        std::stable_sort(rank.begin(), rank.end(), [&](size_t a, size_t b) { return counts[a] > counts[b]; });
+        next.clear();
+        for (size_t i = 0; i < std::min(width, rank.size()); i++) next.push_back(sets[rank[i]]);
+        beam.swap(next);
+    }
+}
+
 bool planBlocksEach(const std::vector<Gate> &gates, int numBits, int tileBits, int seedBits,
                     const std::function<bool(BlockPlan &)> &onBlock, int lookahead) {
     GateDag dag(numBits, true);
@@ -100,7 +132,10 @@ bool planBlocksEach(const std::vector<Gate> &gates, int numBits, int tileBits, i
     while (!dag.empty()) {
         BlockPlan b;
         u64 mask = seed & all;
-        growMask(dag, mask, tileBits, false, look);
+        if (lookahead >= kSearchBeam4)
+            beamMask(dag, mask, tileBits, lookahead == kSearchBeam4 ? 4 : 16);
+        else
+            growMask(dag, mask, tileBits, false, look);
         // pad to tileBits with the lowest unused bits above the seed
         for (int bit = seedBits; popcount64(mask) < tileBits && bit < numBits; bit++) mask |= 1ULL << bit;
         b.tileMask = mask & all;

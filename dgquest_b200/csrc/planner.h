@@ -39,6 +39,10 @@ struct MatrixPool {
     std::vector<std::vector<double>> mats;  // row-major 2^k x 2^k, (re, im) interleaved
 };
 
+// Values of `lookahead` below: -1 by register size, 0 greedy, 1 greedy with a
+// step of lookahead, or a beam search of width 4 or 16.
+constexpr int kSearchBeam4 = 2, kSearchBeam16 = 3;
+
 // `complete` (if given) is set to false when gates are left that no tile
 // can hold (a gate with more non-diagonal targets than the tile width).
 // seedBits: the lowest address bits every tile holds (5: the coalesced bits

@@ -55,13 +55,14 @@ struct QuregState {
     double *dNorm = nullptr;  // complex64 renormalisation: two running sums of |a|^2
 
     int tileBitsSetting = 0;  // 0 = cost model
-    int planLookahead = -1;   // block selection with lookahead (the cost model's choice; -1: by size)
+    int planLookahead = -1;   // block search (the cost model's choice, planner.h; -1: by size)
     bool allowPaired = true;  // complex64: the paired form where it applies
     int denseFusion = -1;     // > 0: gates fused into dense blocks of this many qubits;
                               // -1: the predictor chooses tiles or dense blocks per plan
     double predictedTileSeconds = 0.0;  // the tile-width choice's predicted plan time
     int formTileBits = 0;   // the form choice's tile width for the plan being made (0: none)
     int formLookahead = -1;
+    int formPairedLookahead = -1;  // complex64 paired form: the same choice at its width
     // matrices of the planned dense sweeps (host copy and device buffer)
     std::vector<double> denseHost;
     double *dDense = nullptr;
