@@ -442,7 +442,8 @@ int buildPrograms(QuregState &s, int W, std::vector<TileProgram> &out, PlanStats
                                                  SweepHeader hb = first ? h : SweepHeader();
                                                  const size_t from = out.size();
                                                  if (!encodeBlock(b, s.numBits, s.numQubits, W, s.pool, hb, out, &st,
-                                                                  &err, paired, folds, folds != Folding::None ? &carry : nullptr)) {
+                                                                  &err, paired, folds, folds != Folding::None ? &carry : nullptr,
+                                                                  s.single)) {
                                                      code = E_UNSUPPORTED;
                                                      return false;
                                                  }

@@ -439,36 +439,61 @@ void placeDiagonals(std::vector<Phase> &phases, const TileMap &tm, int tileBits,
                  phases.end());
 }
 
-// Cuts phases whose ops or coefficients could exceed a program's capacity
-// (gates gathered in one phase); the parts keep the phase's layout.
-void splitLongPhases(std::vector<Phase> &phases) {
+// Bits (-log2) by which a gate may shrink the scalar that its sweep leaves to
+// one multiply: the factors of uncontrolled rotations, Hadamards and XY-plane
+// unitaries, and the first entry of a general 2x2 in a framed program.
+double scalarBits(const Gate &g) {
+    if (g.controlMask || isDiagonalType(g.type) || g.type == OP_MULTI_UNITARY) return 0.0;
+    switch (g.type) {
+        case OP_PAULI_X:
+        case OP_PAULI_Y:
+        case OP_PAULI_Y_CONJ: return 0.0;
+        case OP_HADAMARD: return 0.5;
+        case OP_ROTATE_X:
+        case OP_ROTATE_Y: return -std::log2(std::max(std::fabs(std::cos(g.op[0])), std::fabs(std::sin(g.op[0]))));
+        default: {
+            double m[8];
+            gateMatrix(g, m);
+            const double d = std::max(std::hypot(m[0], m[1]), std::hypot(m[4], m[5]));
+            return d > 0.0 && d < 1.0 ? -std::log2(d) : 0.0;
+        }
+    }
+}
+
+// Cuts phases whose ops, coefficients or scalar could exceed a program's
+// capacity (gates gathered in one phase); the parts keep the phase's layout.
+void splitLongPhases(std::vector<Phase> &phases, bool scalarLimited) {
     auto coefs = [](const Gate &g) {
         return g.type == OP_MULTI_UNITARY ? 2 << (2 * g.numMultiTargets) : isDiagonalType(g.type) ? 2 : 8;
     };
     std::vector<Phase> out;
     for (Phase &p : phases) {
         int n = 0, c = 0;
-        bool cut = false;
+        double b = 0.0;
         for (const Gate &g : p.gates) {
             n++;
             c += coefs(g);
+            if (scalarLimited) b += scalarBits(g);
         }
-        cut = n > kMaxOps || c > kMaxCoef;
-        if (!cut) {
+        if (n <= kMaxOps && c <= kMaxCoef && b <= kMaxScalarBitsF32) {
             out.push_back(std::move(p));
             continue;
         }
         Phase part{{}, p.front, p.targetsLocal};
         n = c = 0;
+        b = 0.0;
         for (const Gate &g : p.gates) {
-            if (n + 1 > kMaxOps || c + coefs(g) > kMaxCoef) {
+            const double bits = scalarLimited ? scalarBits(g) : 0.0;
+            if (n + 1 > kMaxOps || c + coefs(g) > kMaxCoef || b + bits > kMaxScalarBitsF32) {
                 out.push_back(part);
                 part.gates.clear();
                 n = c = 0;
+                b = 0.0;
             }
             part.gates.push_back(g);
             n++;
             c += coefs(g);
+            b += bits;
         }
         out.push_back(std::move(part));
     }
@@ -530,7 +555,12 @@ bool framedGates(const std::vector<Gate> &gates) {
 
 bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits, const MatrixPool &pool,
                  const SweepHeader &first, std::vector<TileProgram> &out, PlanStats *stats, std::string *err,
-                 bool paired, Folding folds, std::vector<Gate> *carry) {
+                 bool paired, Folding folds, std::vector<Gate> *carry, bool single) {
+    // (at most half a bit a gate: few blocks can reach the limit)
+    int pairGates = 0;
+    if (single || paired)
+        for (const Gate &g : block.gates) pairGates += !isDiagonalType(g.type) && !g.controlMask;
+    const bool scalarLimited = 0.5 * pairGates > kMaxScalarBitsF32;
     const TileMap tm = makeTileMap(block.tileMask, numBits);
     std::vector<Gate> carried;
     if (carry) carried.swap(*carry);
@@ -591,10 +621,8 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
         }
     }
 
-    if (folds != Folding::None) {
-        placeDiagonals(phases, tm, tileBits, paired, block.last ? nullptr : carry);
-        splitLongPhases(phases);
-    }
+    if (folds != Folding::None) placeDiagonals(phases, tm, tileBits, paired, block.last ? nullptr : carry);
+    if (folds != Folding::None || scalarLimited) splitLongPhases(phases, scalarLimited);
 
     // ---- programs
     auto newProgram = [&](bool isFirst) {
@@ -626,6 +654,7 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
     };
     TileProgram *prog = newProgram(true);
     int numCoef = 0;
+    double scalar = 0.0;  // the program's scalar may have shrunk by so many bits
 
     for (const Phase &ph : phases) {
         const PhaseLayout L = makeLayout(ph.front, ph.targetsLocal, tileBits, paired);
@@ -633,13 +662,14 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
         // rotations leave their scalar factor in (phRe, phIm)
         std::vector<KOp> ops;
         std::vector<double> coef;
-        double phRe = 1.0, phIm = 0.0;
+        double phRe = 1.0, phIm = 0.0, phBits = 0.0;
         auto scaleBy = [&](double fr, double fi) {
             const double r = phRe * fr - phIm * fi, i = phRe * fi + phIm * fr;
             phRe = r;
             phIm = i;
         };
         for (const Gate &g : ph.gates) {
+            if (scalarLimited) phBits += scalarBits(g);
             KOp op;
             std::memset(&op, 0, sizeof(op));
             op.selCta = -1;
@@ -846,10 +876,12 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
         }
         // start a new program (one more sweep over the same tile) when full
         if (prog->numPhases + 1 > kMaxPhases || prog->numOps + (int) ops.size() > kMaxOps ||
-            numCoef + (int) coef.size() > kMaxCoef) {
+            numCoef + (int) coef.size() > kMaxCoef || scalar + phBits > kMaxScalarBitsF32) {
             prog = newProgram(false);
             numCoef = 0;
+            scalar = 0.0;
         }
+        scalar += phBits;
         if (phRe != 1.0 || phIm != 0.0) {
             const double gr = prog->globalRe, gi = prog->globalIm;
             prog->globalRe = gr * phRe - gi * phIm;

@@ -85,9 +85,18 @@ enum class Folding { None, Framed, Specialised };
 // diagonal gates then move to the phases where they are such factors. carry (with folds): diagonal gates of
 // the block before, run first here; the block's own that would be cheaper in
 // the next block are left in it (none when the block is the last).
+// single: a complex64 state. Its kernels apply a program's scalar (the product
+// of the factors that rotations and Hadamards leave out) as one float, before,
+// between or after the ops, so a program ends before it falls below
+// 2^-kMaxScalarBitsF32: amplitudes then grow by at most 2^80 of the 2^127 a
+// float holds, and what drops below its 2^-149 is under 2^-69 of the norm.
+// (640 Hadamards in one sweep leave 2^-320: 0 as a float.) In complex128 the
+// ops of one program cannot leave that range.
+constexpr double kMaxScalarBitsF32 = 80.0;
 bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits, const MatrixPool &pool,
                  const SweepHeader &first, std::vector<TileProgram> &out, PlanStats *stats, std::string *err,
-                 bool paired = false, Folding folds = Folding::None, std::vector<Gate> *carry = nullptr);
+                 bool paired = false, Folding folds = Folding::None, std::vector<Gate> *carry = nullptr,
+                 bool single = false);
 
 // Whether the framed interpreter is likely to run every gate (frame.h; a
 // general 2x2 without controls may still turn out to have no framed form,
