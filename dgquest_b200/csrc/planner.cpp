@@ -622,7 +622,7 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
     }
 
     if (folds != Folding::None) placeDiagonals(phases, tm, tileBits, paired, block.last ? nullptr : carry);
-    if (folds != Folding::None || scalarLimited) splitLongPhases(phases, scalarLimited);
+    splitLongPhases(phases, scalarLimited);
 
     // ---- programs
     auto newProgram = [&](bool isFirst) {

@@ -79,3 +79,36 @@ def test_batches_with_and_without_a_framed_form(quest, env, unframed):
             Q.destroyQureg(q, env)
     for n, ops, a in zip(sizes, lists, states):
         check(a, oracle.run(n, ops)[0], False)
+
+
+@pytest.mark.parametrize("unframed", [False, True])
+def test_a_phase_longer_than_a_program(quest, env, unframed):
+    # 1050 gates on 4 qubits: one register phase, cut into two programs; the
+    # same register in a batch
+    Q, n = quest, 4
+    b = C.OpList()
+    for _ in range(150):
+        for t in range(n):
+            b.add(C.H, t)
+        for t in range(n - 1):
+            b.add(C.CZ, t, t + 1)
+    if unframed:
+        b.add(C.CRX, 0, 1, p=(0.3,))
+    ops = b.array()
+    ref = oracle.run(n, ops)[0]
+    for batched in (False, True):
+        q = Q.createQureg(n, env)
+        try:
+            Q.dgq_setTileBits(q, 9)
+            Q.dgq_setDenseFusion(q, 0)
+            C.replay(q, ops)
+            if batched:
+                batch = Q.Batch([q], config={"tileBits": 12})
+                batch.launch()
+                batch.wait()
+            amps = Q.state_vector(q)
+            if batched:
+                batch.close()
+        finally:
+            Q.destroyQureg(q, env)
+        check(amps, ref, False)

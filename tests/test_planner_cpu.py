@@ -2,6 +2,10 @@
 the headline circuits, DAG merge rules, and NVRTC compiles of generated
 sweep kernels for sm_100a (no GPU is used)."""
 import ctypes
+import os
+import subprocess
+import sys
+import tempfile
 
 import numpy as np
 import pytest
@@ -11,6 +15,7 @@ from dgquest_b200 import ir
 from dgquest_b200 import quest as Q
 
 P = ctypes.POINTER
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def test_random_circuit_plan_shape():
@@ -123,3 +128,32 @@ def test_specialise_ahead_counts_the_plans_kernels():
     assert count == ir.plan(ops, n, 0).sweeps
     with pytest.raises(Q.QuESTError):
         Q.dgq_specialiseGates(n, 4, 0, None, None, None, None, 1)
+
+
+def long_phase(n=4, layers=150, unframed=False):
+    b = C.OpList()
+    for d in range(layers):
+        for q in range(n):
+            b.add(C.H, q)
+        for q in range(n - 1):
+            b.add(C.CZ, q, q + 1)
+    if unframed:
+        b.add(C.CRX, 0, 1, p=(0.3,))
+    return b.array()
+
+
+@pytest.mark.parametrize("unframed", [False, True])
+def test_a_phase_longer_than_a_program_is_cut(unframed):
+    # 1050 gates on 4 qubits are one register phase of a one-tile register;
+    # a program holds 640 ops
+    ops = long_phase(unframed=unframed)
+    code = ("import sys; sys.path.insert(0, sys.argv[1]); import numpy as np\n"
+            "from dgquest_b200 import ir\n"
+            "print(ir.plan(np.load(sys.argv[2]), 4, 9).sweeps)")
+    with tempfile.TemporaryDirectory() as d:
+        np.save(os.path.join(d, "ops.npy"), ops)
+        for jit in ("0", "1"):
+            r = subprocess.run([sys.executable, "-c", code, ROOT, os.path.join(d, "ops.npy")], capture_output=True,
+                               text=True, env={**os.environ, "DGQ_JIT": jit}, timeout=300)
+            assert r.returncode == 0, r.stderr[-1000:]
+            assert int(r.stdout) == 2
