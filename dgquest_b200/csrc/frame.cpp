@@ -10,12 +10,17 @@ namespace {
 
 int parity(uint32_t x) { return __builtin_parity(x); }
 
+// bit j: parity of j & r
+uint32_t parityTable(uint32_t r) {
+    return ((r & 1u) ? 0xAAAAu : 0u) ^ ((r & 2u) ? 0xCCCCu : 0u) ^ ((r & 4u) ? 0xF0F0u : 0u) ^ ((r & 8u) ? 0xFF00u : 0u);
+}
+
 struct Framer {
     const TileProgram &p;
     FrameSweep &out;
     const KPhase *ph = nullptr;
     // register bits: value = row . j + dl . loc + dc . cta + cc
-    uint8_t row[kRegBits];
+    uint8_t row[kRegBits], col[kRegBits];  // M and its inverse, whose column q is the direction of a pair on bit q
     uint16_t dl[kRegBits];
     uint32_t dc[kRegBits];
     uint8_t cc[kRegBits];
@@ -96,32 +101,46 @@ struct Framer {
             put(op, c, s);
             return true;
         }
-        if (n > 2 || condLoc || condCta) return false;
-        const int a = __builtin_ctz(regs), b = 31 - __builtin_clz(regs);
-        op.code = (uint8_t) ((neg ? FK_NEG2 : FK_PH2) << 4);
-        op.rr = (uint8_t) (row[a] | row[b] << 4);
-        op.tab = (uint16_t) (cc[a] | cc[b] << 1);
-        op.lm = dl[a];
-        op.cm = dc[a];
-        op.lm2 = dl[b];
-        op.cm2 = dc[b];
-        put(op, c, s);
+        if (condLoc || condCta) {
+            op.code = (uint8_t) (FK_IF << 4);
+            op.lm = (uint16_t) condLoc;
+            op.cm = condCta;
+            put(op, 0.0, 0.0);
+        }
+        // two register bits at a time, the last two with the phase
+        uint32_t left = regs;
+        while (left) {
+            const int k = __builtin_popcount(left);
+            const int a = __builtin_ctz(left), b = k == 3 ? -1 : __builtin_ctz(left & (left - 1));
+            std::memset(&op, 0, sizeof(op));
+            op.code = (uint8_t) ((k > 2 ? FK_AND : neg ? FK_NEG2 : FK_PH2) << 4);
+            op.rr = row[a];
+            op.tab = cc[a];
+            op.lm = dl[a];
+            op.cm = dc[a];
+            if (b < 0) {
+                op.tab |= 2;  // always 1
+            } else {
+                op.rr |= (uint8_t) (row[b] << 4);
+                op.tab |= (uint16_t) (cc[b] << 1);
+                op.lm2 = dl[b];
+                op.cm2 = dc[b];
+                left &= left - 1;
+            }
+            left &= left - 1;
+            put(op, c, s);
+        }
         return true;
     }
     // rotation on register bit q; (a, b) its coefficients
     void pair(int kind, int q, double a, double b) {
-        int v = 0;
-        for (int j = 1; j < kRegs && !v; j++) {
-            bool hit = true;
-            for (int r = 0; r < kRegBits; r++) hit = hit && parity(row[r] & j) == (r == q);
-            if (hit) v = j;
-        }
+        const int v = col[q];
         FOp op;
         std::memset(&op, 0, sizeof(op));
         op.code = (uint8_t) (kind << 4 | v);
         if (kind != FK_RX) {
             // Rx is the same both ways round
-            for (int j = 0; j < kRegs; j++) op.tab |= (uint16_t) ((parity(row[q] & j) ^ cc[q]) << j);
+            op.tab = (uint16_t) (parityTable(row[q]) ^ (cc[q] ? 0xFFFFu : 0u));
             op.lm = dl[q];
             op.cm = dc[q];
         }
@@ -171,6 +190,7 @@ struct Framer {
                 } else if (k.ctrlReg) {
                     const int s = __builtin_ctz(k.ctrlReg);
                     row[q] ^= row[s];
+                    col[s] ^= col[q];
                     dl[q] ^= dl[s];
                     dc[q] ^= dc[s];
                     cc[q] ^= cc[s];
@@ -240,7 +260,7 @@ struct Framer {
         uint32_t regMask = 0;
         zr = 0;
         for (int b = 0; b < kRegBits; b++) {
-            row[b] = (uint8_t) (1u << b);
+            row[b] = col[b] = (uint8_t) (1u << b);
             dl[b] = 0;
             dc[b] = 0;
             cc[b] = 0;
@@ -258,11 +278,12 @@ struct Framer {
         FPhase f;
         std::memset(&f, 0, sizeof(f));
         for (int i = 0; i < W - kRegBits; i++) f.thrPos[i] = kp.thrPos[i];
+        uint32_t table[kRegBits];
+        for (int b = 0; b < kRegBits; b++) table[b] = parityTable(row[b]) ^ (cc[b] ? 0xFFFFu : 0u);
         for (int j = 0; j < kRegs; j++) {
             f.rdOff[j] = kp.regOff[j];
             uint32_t loc = 0;
-            for (int b = 0; b < kRegBits; b++)
-                if (parity(row[b] & j) ^ cc[b]) loc |= 1u << kp.regPos[b];
+            for (int b = 0; b < kRegBits; b++) loc |= ((table[b] >> j) & 1u) << kp.regPos[b];
             f.wrOff[j] = (uint16_t) tileSwizzle(loc);
         }
         for (int b = 0; b < kRegBits; b++) {
@@ -282,12 +303,7 @@ struct Framer {
         out.phases.push_back(f);
         // the sign in index bits: zr . j = m . (M j)
         uint32_t m = 0;
-        for (uint32_t t = 0; t < (uint32_t) kRegs; t++) {
-            uint32_t r = 0;
-            for (int b = 0; b < kRegBits; b++)
-                if ((t >> b) & 1u) r ^= row[b];
-            if (r == zr) m = t;
-        }
+        for (int b = 0; b < kRegBits; b++) m |= (uint32_t) parity(zr & col[b]) << b;
         signLoc = zl;
         for (int b = 0; b < kRegBits; b++)
             if ((m >> b) & 1u) {
@@ -306,6 +322,9 @@ bool frameProgram(const TileProgram &p, int W, FrameSweep &out) {
     out.ops.clear();
     out.coef.clear();
     if (p.paired || p.denseK || W > kMaxTileBitsF64 || p.numBits - W > 32) return false;
+    out.phases.reserve((size_t) p.numPhases);
+    out.ops.reserve((size_t) p.numOps + 16);
+    out.coef.reserve(2 * (size_t) p.numOps + 32);
     Framer f(p, out);
     uint32_t signLoc = 0;
     for (int i = 0; i < p.numPhases; i++)
@@ -362,6 +381,7 @@ void applyFramedHost(const TileProgram &p, const FrameSweep &f, int W, double *s
                 for (int i = 0; i < W - kRegBits; i++) loc |= ((tid >> i) & 1u) << ph.thrPos[i];
                 const uint32_t sb = tileSwizzle(loc);
                 double a[kRegs][2], acc[2] = {1.0, 0.0};
+                uint32_t where = 0xFFFFu;  // registers left by FK_AND and FK_IF
                 if (f.tail.globalPhase >= 0 && &ph == &f.phases[(size_t) f.tail.globalPhase]) {
                     acc[0] = f.tail.globalRe;
                     acc[1] = f.tail.globalIm;
@@ -394,12 +414,18 @@ void applyFramedHost(const TileProgram &p, const FrameSweep &f, int W, double *s
                         if ((loc & op.lm2) != op.lm2 || (cta & op.cm2) != op.cm2) continue;
                         for (int j = 0; j < kRegs; j++)
                             if (parity(j & v) ^ thr) mul(a[j], c0, c1);
+                    } else if (kind == FK_IF) {
+                        if ((loc & op.lm) != op.lm || (cta & op.cm) != op.cm) where = 0;
                     } else {
                         const int thr2 = parity(loc & op.lm2) ^ parity(cta & op.cm2);
                         for (int j = 0; j < kRegs; j++)
-                            if ((parity(j & (op.rr & 15)) ^ thr ^ (op.tab & 1)) &
-                                (parity(j & (op.rr >> 4)) ^ thr2 ^ ((op.tab >> 1) & 1)))
-                                mul(a[j], c0, c1);
+                            if (!((parity(j & (op.rr & 15)) ^ thr ^ (op.tab & 1)) &
+                                  (parity(j & (op.rr >> 4)) ^ thr2 ^ ((op.tab >> 1) & 1))))
+                                where &= ~(1u << j);
+                        if (kind == FK_AND) continue;
+                        for (int j = 0; j < kRegs; j++)
+                            if ((where >> j) & 1u) mul(a[j], c0, c1);
+                        where = 0xFFFFu;
                     }
                 }
                 uint32_t wb = sb;

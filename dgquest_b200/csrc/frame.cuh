@@ -109,6 +109,7 @@ __device__ __forceinline__ void framePhases(int numPhases, const FrameTail &tail
         const bool start = p == tail.globalPhase;
         double ar = start ? tail.globalRe : 1.0, ai = start ? tail.globalIm : 0.0;
         const int se = ph.scalarEnd, e = ph.opEnd;
+        uint32_t where = 0xFFFFu;  // registers left by FK_AND and FK_IF
         for (int o = ph.opBegin; o < se; o++) {
             const FOp op = fetchOp(o);
             const double2 c = fetchCoef(o);
@@ -149,9 +150,15 @@ __device__ __forceinline__ void framePhases(int numPhases, const FrameTail &tail
                     DGQ_FRAME_CASES(FK_NEG, (frameNegate<D>(a)))
                 }
             } else {
-                uint32_t m = parityTable(op.rr & 15u) ^ ((op.tab & 1u) ? 0xFFFFu : 0u) ^ (thr ? 0xFFFFu : 0u);
+                if (op.code == FK_IF << 4) {
+                    if ((loc & op.lm) != op.lm || (cta & op.cm) != op.cm) where = 0u;
+                    continue;
+                }
+                uint32_t m = where & (parityTable(op.rr & 15u) ^ ((op.tab & 1u) ? 0xFFFFu : 0u) ^ (thr ? 0xFFFFu : 0u));
                 const uint32_t thr2 = (uint32_t) (__popc(loc & op.lm2) + __popc(cta & op.cm2)) & 1u;
                 m &= parityTable(op.rr >> 4) ^ ((op.tab & 2u) ? 0xFFFFu : 0u) ^ (thr2 ? 0xFFFFu : 0u);
+                where = op.code == FK_AND << 4 ? m : 0xFFFFu;
+                if (op.code == FK_AND << 4) continue;
                 if (op.code == FK_NEG2 << 4) {
 #pragma unroll
                     for (int j = 0; j < kRegs; j++) {

@@ -23,7 +23,11 @@
 // a register of one tile waits mostly for instruction fetches. Measured
 // against the form with CNOT operations: a batch of 48 registers of 10..20
 // qubits 5.30 -> 4.25 ms, the five sweeps of a 21-qubit Fourier transform
-// 248 -> 190 us, one tile of a 10-qubit ansatz 33.9 -> 26.8 us.
+// 248 -> 190 us, one tile of a 10-qubit ansatz 33.9 -> 26.8 us. Phases on three
+// qubits and more are chains of records (a list that held one ran on the
+// general interpreter before): 12 rotation layers with four of them each, 14
+// and 20 qubits, 215 -> 179 and 439 -> 408 us; 48 such registers of 10..18
+// qubits in a batch 1335 -> 1147 us, one such among 48 944 -> 694 us.
 #pragma once
 
 #include <cstdint>
@@ -43,17 +47,21 @@ enum FrameKind : uint8_t {
     FK_NEG = 4,   // the same with -1
     FK_PH2 = 5,   // (c + i s) where two such parities are 1
     FK_NEG2 = 6,
+    // before an FK_PH2 or FK_NEG2, for phases on three or four register bits
+    // or under a thread or CTA condition:
+    FK_AND = 7,   // and where two more such parities are 1
+    FK_IF = 8,    // and where every bit of the condition lm, cm is 1
 };
 
 // 16 bytes, read uniformly.
 struct FOp {
     uint8_t code;
-    uint8_t rr;    // FK_PH2 / FK_NEG2: parity mask of j of the first (low 4 bits) and second functional
-    uint16_t tab;  // pair ops: bit j = parity of j (and the constant); FK_*2: bits 0, 1 the constants
+    uint8_t rr;    // FK_*2, FK_AND: parity mask of j of the first (low 4 bits) and second functional
+    uint16_t tab;  // pair ops: bit j = parity of j (and the constant); FK_*2, FK_AND: bits 0, 1 the constants
     uint16_t lm, lm2;  // thread bits (tile-local) and
     uint32_t cm, cm2;  // CTA bits: pair ops and FK_PH / FK_NEG: parity masks lm, cm, condition lm2, cm2
-                       // (all ones); FK_*2: parity masks of the first and second functional;
-                       // scalar ops: condition lm, cm
+                       // (all ones); FK_*2, FK_AND: parity masks of the first and second functional;
+                       // FK_IF and scalar ops: condition lm, cm
 };
 static_assert(sizeof(FOp) == 16, "FOp layout");
 
@@ -109,8 +117,7 @@ struct FrameSweep {
 
 // The framed form of a tile program of width W (unpaired, W <= 12); false
 // when an op has none (dense ops, controlled rotations and general 2x2 ops,
-// controlled Y, X with several controls, 2x2 matrices unitary only to 1e-14, phases on three register bits or on
-// two under a thread control).
+// controlled Y, X with several controls, 2x2 matrices unitary only to 1e-14).
 bool frameProgram(const TileProgram &p, int W, FrameSweep &out);
 
 // The sweep on the host, on 2^numBits amplitudes (re, im pairs).

@@ -543,6 +543,9 @@ void encodeHeaderOnly(int numBits, int numReal, int tileBits, const SweepHeader 
     for (int i = 0; i < numBits - tileBits; i++) out.ctaPos[i] = (uint8_t) (tileBits + i);
 }
 
+// (Phases on three qubits and more have a framed form too, but placing the
+// diagonal gates of such lists costs more on the host, 50 us of 770 at 14
+// qubits, than it saves on the GPU, 5 us of 179.)
 bool framedGates(const std::vector<Gate> &gates) {
     for (const Gate &g : gates) {
         const int controls = popcount64(g.controlMask);

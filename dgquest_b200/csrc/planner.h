@@ -98,10 +98,10 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
                  bool paired = false, Folding folds = Folding::None, std::vector<Gate> *carry = nullptr,
                  bool single = false);
 
-// Whether the framed interpreter is likely to run every gate (frame.h; a
-// general 2x2 without controls may still turn out to have no framed form,
-// and then runs on the other interpreter, which runs any plan but the
-// specialised kernels').
+// Whether the framed interpreter is likely to run every gate (frame.h) and
+// placing diagonal gates for it pays (a general 2x2 without controls may still
+// turn out to have no framed form, and then runs on the other interpreter,
+// which runs any plan but the specialised kernels').
 bool framedGates(const std::vector<Gate> &gates);
 
 // A program that only applies the header (init and/or lazy collapse).

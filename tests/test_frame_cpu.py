@@ -44,3 +44,39 @@ def test_gates_without_a_framed_form_are_refused(kind):
     ops = np.concatenate([C.hea(10, 1, 3), C.mixed_ops(10, 3, 5, kinds=[kind])])
     got, sweeps = framed(10, 10, ops)
     assert sweeps == 0 and got[0] == 1.0 and not got[1:].any()
+
+
+def multi_controlled(n, seed, rounds=6):
+    """Rotations and CNOT, then phases and sign flips on 3 qubits and more:
+    (IR arrays, the oracle's state)."""
+    gen = np.random.default_rng(seed)
+    o = oracle.Oracle(n)
+    parts = []
+    for r in range(rounds):
+        ops = C.mixed_ops(n, 25, seed + r, kinds=[C.H, C.RX, C.RY, C.RZ, C.CNOT, C.CNOT, C.X, C.UNITARY])
+        parts.append(ir.ops_to_ir(ops, n))
+        o.apply(ops)
+        for _ in range(4):
+            qubits = gen.choice(n, gen.integers(3, min(n, 7) + 1), replace=False)
+            mask = sum(1 << int(q) for q in qubits)
+            kind = [ir.OP_Z, ir.OP_PHASE, ir.OP_S][gen.integers(3)]
+            angle = gen.uniform(-3, 3)
+            parts.append((np.array([kind], dtype=np.int32), np.array([0], dtype=np.uint64),
+                          np.array([mask], dtype=np.uint64), np.array([[angle] + 7 * [0.0]])))
+            a = o.amps()
+            a[(np.arange(1 << n) & mask) == mask] *= {ir.OP_Z: -1, ir.OP_S: 1j}.get(kind, np.exp(1j * angle))
+            o.set_amps(a)
+    want = o.amps()
+    o.close()
+    return [np.concatenate(x) for x in zip(*parts)], want
+
+
+@pytest.mark.parametrize("n,w", [(9, 9), (12, 9), (11, 10), (13, 11), (12, 12), (14, 12)])
+@pytest.mark.parametrize("seed", range(4))
+def test_phases_on_many_qubits_are_framed(n, w, seed):
+    arrays, want = multi_controlled(n, 100 * n + seed)
+    a = np.zeros(1 << n, dtype=np.complex128)
+    a[0] = 1.0
+    got, sweeps = ir.frame_apply_host(n, w, *arrays, a)
+    assert sweeps >= 1
+    assert np.abs(got - want).max() <= 1e-12

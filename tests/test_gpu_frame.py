@@ -112,3 +112,46 @@ def test_a_phase_longer_than_a_program(quest, env, unframed):
         finally:
             Q.destroyQureg(q, env)
         check(amps, ref, False)
+
+
+@pytest.mark.parametrize("single", [False, True])
+@pytest.mark.parametrize("n,width", [(6, 9), (10, 9), (13, 11), (14, 12)])
+def test_phases_on_many_qubits(quest, env, n, width, single):
+    # phases and sign flips on 3..6 qubits among rotations and CNOT, by itself
+    # and in a batch with a register that has none
+    Q, gen = quest, np.random.default_rng(n)
+    o = oracle.Oracle(n)
+    regs = [(Q.dgq_createQuregF32 if single else Q.createQureg)(n, env) for _ in range(3)]
+    try:
+        for q in regs:
+            Q.dgq_setTileBits(q, width)
+            Q.dgq_setDenseFusion(q, 0)
+        for r in range(5):
+            ops = C.mixed_ops(n, 20, 7 * n + r, kinds=[C.H, C.RX, C.RY, C.RZ, C.CNOT, C.CNOT, C.X, C.UNITARY])
+            o.apply(ops)
+            for q in regs:
+                Q.apply_circuit(q, ops)
+            for _ in range(3):
+                k = int(gen.integers(3, 7))
+                qubits = gen.choice(n, k, replace=False).tolist()
+                flip, angle = bool(gen.integers(2)), float(gen.uniform(-3, 3))
+                a = o.amps()
+                mask = sum(1 << t for t in qubits)
+                a[(np.arange(1 << n) & mask) == mask] *= -1 if flip else np.exp(1j * angle)
+                o.set_amps(a)
+                for q in regs[:2]:
+                    if flip:
+                        Q.multiControlledPhaseFlip(q, Q.int_array(qubits), k)
+                    else:
+                        Q.multiControlledPhaseShift(q, Q.int_array(qubits), k, angle)
+        want = o.amps()
+        o.close()
+        check(Q.state_vector(regs[0]), want, single)
+        b = Q.Batch(regs[1:], config={"tileBits": width})
+        b.launch()
+        b.wait()
+        check(Q.state_vector(regs[1]), want, single)
+        b.close()
+    finally:
+        for q in regs:
+            Q.destroyQureg(q, env)
