@@ -14,7 +14,7 @@ extern "C" {
 // superoperator S[(r', c')][(r, c)] = sum_K K[r'][r] conj(K[c'][c]).
 using Kraus = std::vector<std::complex<double>>;  // d x d, row-major
 
-static void recordChannel(Qureg q, const int *qs, int k, const std::vector<Kraus> &kraus) {
+static void recordChannel(Qureg q, const int *qs, int k, const std::vector<Kraus> &kraus, dgq::MatrixShape shape) {
     QuregState &s = *stateOf(q);
     const int n = s.densityQubits, d = 1 << k, D = d * d;
     std::vector<double> m((size_t) 2 * D * D, 0.0);
@@ -35,6 +35,7 @@ static void recordChannel(Qureg q, const int *qs, int k, const std::vector<Kraus
     g.targetMask = toVirtualMask(s, tm);
     g.controlMask = 0;
     g.numMultiTargets = 2 * k;
+    g.multiShape = shape;
     for (int i = 0; i < k; i++) {
         g.multiTargets[i] = s.l2v[qs[i]];
         g.multiTargets[k + i] = s.l2v[qs[i] + n];
@@ -82,7 +83,7 @@ void applyOneQubitDephaseError(Qureg q, const int targetQubit, qreal prob) {
     Kraus K0 = pauli(0), K1 = pauli(3);
     for (auto &x : K0) x *= a;
     for (auto &x : K1) x *= b;
-    recordChannel(q, &targetQubit, 1, {K0, K1});
+    recordChannel(q, &targetQubit, 1, {K0, K1}, dgq::SHAPE_DIAGONAL);
 }
 
 // include/QuEST.h:1399: (1 - p) rho + p/3 (Za rho Za + Zb rho Zb + ZaZb rho ZaZb)
@@ -93,7 +94,8 @@ void applyTwoQubitDephaseError(Qureg q, const int qubit1, const int qubit2, qrea
     const int qs[2] = {qubit1, qubit2};
     const double w = std::sqrt(prob / 3.0);
     recordChannel(q, qs, 2,
-                  {pauli2(0, 0, std::sqrt(1.0 - prob)), pauli2(3, 0, w), pauli2(0, 3, w), pauli2(3, 3, w)});
+                  {pauli2(0, 0, std::sqrt(1.0 - prob)), pauli2(3, 0, w), pauli2(0, 3, w), pauli2(3, 3, w)},
+                  dgq::SHAPE_DIAGONAL);
 }
 
 // include/QuEST.h:1423: (1 - p) rho + p/3 (X rho X + Y rho Y + Z rho Z)
@@ -106,7 +108,7 @@ void applyOneQubitDepolariseError(Qureg q, const int targetQubit, qreal prob) {
         for (auto &x : K) x *= w;
         ks.push_back(K);
     }
-    recordChannel(q, &targetQubit, 1, ks);
+    recordChannel(q, &targetQubit, 1, ks, dgq::SHAPE_DEPOLARISE);
 }
 
 // include/QuEST.h:1445: amplitude damping (decay to |0>) with probability p:
@@ -116,7 +118,7 @@ void applyOneQubitDampingError(Qureg q, const int targetQubit, qreal prob) {
     if (!vNoise(q, targetQubit, prob, 1.0, E_INVALID_PROB, __func__)) return;
     const Kraus K0 = {1.0, 0.0, 0.0, std::sqrt(1.0 - prob)};
     const Kraus K1 = {0.0, std::sqrt(prob), 0.0, 0.0};
-    recordChannel(q, &targetQubit, 1, {K0, K1});
+    recordChannel(q, &targetQubit, 1, {K0, K1}, dgq::SHAPE_DAMPING);
 }
 
 // include/QuEST.h:1494: (1 - p) rho + p/15 (sum of the 15 non-identity
@@ -130,7 +132,7 @@ void applyTwoQubitDepolariseError(Qureg q, const int qubit1, const int qubit2, q
     for (int pa = 0; pa < 4; pa++)
         for (int pb = 0; pb < 4; pb++)
             ks.push_back(pauli2(pa, pb, pa == 0 && pb == 0 ? std::sqrt(1.0 - prob) : std::sqrt(prob / 15.0)));
-    recordChannel(q, qs, 2, ks);
+    recordChannel(q, qs, 2, ks, dgq::SHAPE_DEPOLARISE);
 }
 
 // include/QuEST.h:1507: combineQureg := (1 - prob) combineQureg + prob

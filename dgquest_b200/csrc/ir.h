@@ -45,6 +45,16 @@ enum GateType : int {
 
 static inline bool isDiagonalType(int t) { return t < OP_PAULI_X; }
 
+// Which entries of an OP_MULTI_UNITARY matrix can differ from zero, whatever
+// the numbers: all, or those of a noise channel's superoperator on the row
+// qubits (low half of the targets) and column qubits (high half).
+enum MatrixShape : int32_t {
+    SHAPE_FULL = 0,
+    SHAPE_DIAGONAL = 1,    // dephasing
+    SHAPE_DEPOLARISE = 2,  // the diagonal, and every pair of indices with row = column
+    SHAPE_DAMPING = 3,     // the diagonal, and |1><1| -> |0><0| (two targets)
+};
+
 struct Gate {
     GateType type = OP_ONE;
     u64 targetMask = 0;
@@ -56,6 +66,7 @@ struct Gate {
     int32_t multiIndex = -1;  // OP_MULTI_UNITARY: index into the matrix pool
     int32_t multiTargets[8] = {0, 0, 0, 0, 0, 0, 0, 0};  // OP_MULTI_UNITARY target order
     int32_t numMultiTargets = 0;
+    int32_t multiShape = SHAPE_FULL;  // MatrixShape
 
     double angle() const { return op[0]; }
     void setAngle(double a) { op[0] = a; }

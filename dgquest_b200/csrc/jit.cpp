@@ -1,5 +1,6 @@
 // jit.cpp -- see jit.h.
 #include "jit.h"
+#include "ir.h"
 
 #include <nvrtc.h>
 
@@ -33,31 +34,30 @@ const char *kernelKindName(int code) {
 }
 
 // The entries of a dense op's matrix that take part, as a type for jDenseAt:
-// re(i) / im(i) whether the part of entry i is non-zero, same(r) whether row r
-// is exactly a row of the identity. `m`: the coefficients, 2^k x 2^k (re, im).
-std::string densePattern(const double *m, int k) {
-    const int D = 1 << k;
+// re(i) / im(i) whether the real / imaginary part of entry i can differ from
+// zero. It follows from the kind of the gate, not from its numbers: patterns
+// taken from the matrices made a kernel for every set of zeros that random
+// Paulis, or a channel of another probability, happened to have.
+std::string densePattern(int shape, int k) {
+    const int D = 1 << k, d = 1 << (k / 2);
     uint64_t re[4] = {0}, im[4] = {0};
-    unsigned same = 0;
-    for (int r = 0; r < D; r++) {
-        bool identity = true;
+    for (int r = 0; r < D; r++)
         for (int c = 0; c < D; c++) {
             const int i = r * D + c;
-            if (m[2 * i] != 0.0) re[i >> 6] |= 1ULL << (i & 63);
-            if (m[2 * i + 1] != 0.0) im[i >> 6] |= 1ULL << (i & 63);
-            identity = identity && m[2 * i] == (r == c ? 1.0 : 0.0) && m[2 * i + 1] == 0.0;
+            auto paired = [&](int x) { return x % d == x / d; };  // row = column
+            const bool on = shape == SHAPE_FULL || r == c || (shape == SHAPE_DEPOLARISE && paired(r) && paired(c)) ||
+                            (shape == SHAPE_DAMPING && r == 0 && c == D - 1);
+            if (on) re[i >> 6] |= 1ULL << (i & 63);
+            if (on && shape == SHAPE_FULL) im[i >> 6] |= 1ULL << (i & 63);
         }
-        if (identity) same |= 1u << r;
-    }
     std::ostringstream o;
     o << "dgq::DensePattern<";
-    for (uint64_t w : re) o << w << "ull, ";
-    for (uint64_t w : im) o << w << "ull, ";
-    o << same << "u>";
+    for (int w = 0; w < 4; w++) o << re[w] << "ull, ";
+    for (int w = 0; w < 4; w++) o << im[w] << (w < 3 ? "ull, " : "ull>");
     return o.str();
 }
 
-void emitOp(std::ostringstream &o, const KOp &op, const double *coefs) {
+void emitOp(std::ostringstream &o, const KOp &op) {
     const unsigned cr = op.ctrlReg;
     const int off = op.coef;
     std::ostringstream body;
@@ -97,11 +97,9 @@ void emitOp(std::ostringstream &o, const KOp &op, const double *coefs) {
         body << "dgq::jMULNI<" << (op.code == KC_MULNI + 1 ? "true" : "false") << ", " << cr << "u>(a);";
     } else if (op.code >= KC_DENSE && op.code < KC_DENSE + 4) {
         const int k = op.code - KC_DENSE + 1;
-        if (op.selLoc & kDenseAnyBits)
-            body << "dgq::jDenseAt<" << k << ", " << (op.selLoc & 0xFF) << "u, " << densePattern(coefs + off, k)
-                 << ">(a, prog.coef + " << off << ");";
-        else
-            body << "dgq::jDense<" << k << ", " << cr << "u>(a, prog.coef + " << off << ");";
+        const bool any = (op.selLoc & kDenseAnyBits) != 0;  // else register bits 0..k-1
+        body << "dgq::jDenseAt<" << k << ", " << (any ? op.selLoc & 0xFF : 0xE4) << "u, "
+             << densePattern(any ? (op.selLoc >> 8) & 3 : SHAPE_FULL, k) << ">(a, prog.coef + " << off << ");";
     } else if (op.code >= KC_RY1 && op.code < KC_H1) {
         static const char *names[4] = {"jRY1", "jRY2", "jRX1", "jRX2"};
         body << "dgq::" << names[(op.code - KC_RY1) / 4] << "<" << (op.code - KC_RY1) % 4 << ">(a, prog.coef + " << off
@@ -920,7 +918,7 @@ std::string generateSweepSource(const TileProgram &prog, int W) {
             if (fold && scalarKind(prog.ops[k]))
                 emitScalarAcc(o, prog.ops[k]);
             else
-                emitOp(o, prog.ops[k], prog.coef);
+                emitOp(o, prog.ops[k]);
         }
         if (fold) o << "    dgq::jGlobal(a, acc_.x, acc_.y);\n";
         if (writeSmem) {
@@ -949,8 +947,7 @@ std::string generateSweepSource(const TileProgram &prog, int W) {
 
 std::string sweepKey(const TileProgram &prog, int W) {
     // the phases and ops whole, and the header fields that choose code; the
-    // other fields and the coefficients are read at run time, except for
-    // which entries of a dense op on any register bits are zero
+    // other fields and the coefficients are read at run time
     const int32_t head[10] = {W,         prog.numPhases, prog.numOps,   prog.initKind,  prog.hasRestrict != 0,
                               prog.hasGlobal, prog.isSingle,  prog.renormIn, prog.renormOut, prog.paired};
     std::string key;
@@ -958,9 +955,6 @@ std::string sweepKey(const TileProgram &prog, int W) {
     key.append(reinterpret_cast<const char *>(head), sizeof(head));
     key.append(reinterpret_cast<const char *>(prog.phases), (size_t) prog.numPhases * sizeof(KPhase));
     key.append(reinterpret_cast<const char *>(prog.ops), (size_t) prog.numOps * sizeof(KOp));
-    for (int i = 0; i < prog.numOps; i++)
-        if (prog.ops[i].kind == KOP_DENSE && (prog.ops[i].selLoc & kDenseAnyBits))
-            key += densePattern(prog.coef + prog.ops[i].coef, prog.ops[i].k);
     return key;
 }
 

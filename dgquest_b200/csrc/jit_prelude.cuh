@@ -270,42 +270,14 @@ __device__ __forceinline__ void jGlobal(V (&a)[kRegs], double grd, double gid) {
     }
 }
 
-template <int KK, uint32_t CR, class V>
-__device__ __forceinline__ void jDense(V (&a)[kRegs], const double *m) {
-    constexpr int D = 1 << KK;
-#pragma unroll
-    for (int g = 0; g < (kRegs >> KK); g++) {
-        const int base = g << KK;
-        if ((base & CR) != CR) continue;
-        V v[D];
-#pragma unroll
-        for (int c = 0; c < D; c++) v[c] = a[base + c];
-#pragma unroll
-        for (int r = 0; r < D; r++) {
-            DGQJ_R re = 0, im = 0;
-#pragma unroll
-            for (int c = 0; c < D; c++) {
-                const DGQJ_R mr = (DGQJ_R) m[2 * (r * D + c)], mi = (DGQJ_R) m[2 * (r * D + c) + 1];
-                re = fma(mr, v[c].x, re);
-                re = fma(-mi, v[c].y, re);
-                im = fma(mr, v[c].y, im);
-                im = fma(mi, v[c].x, im);
-            }
-            a[base + r] = DGQJ_MK(re, im);
-        }
-    }
-}
-
 // Which entries of a dense op's matrix take part (words of 64 entries, row-major).
-template <uint64_t R0, uint64_t R1, uint64_t R2, uint64_t R3, uint64_t I0, uint64_t I1, uint64_t I2, uint64_t I3,
-          uint32_t SAME>
+template <uint64_t R0, uint64_t R1, uint64_t R2, uint64_t R3, uint64_t I0, uint64_t I1, uint64_t I2, uint64_t I3>
 struct DensePattern {
     static __device__ __forceinline__ constexpr bool at(uint64_t w0, uint64_t w1, uint64_t w2, uint64_t w3, int i) {
         return (((i >> 6) == 0 ? w0 : (i >> 6) == 1 ? w1 : (i >> 6) == 2 ? w2 : w3) >> (i & 63)) & 1u;
     }
     static __device__ __forceinline__ constexpr bool re(int i) { return at(R0, R1, R2, R3, i); }
     static __device__ __forceinline__ constexpr bool im(int i) { return at(I0, I1, I2, I3, i); }
-    static __device__ __forceinline__ constexpr bool same(int r) { return (SAME >> r) & 1u; }
 };
 
 // Dense op with matrix bit i on register bit (POS >> 2 i) & 3, only the
@@ -327,7 +299,6 @@ __device__ __forceinline__ void jDenseAt(V (&a)[kRegs], const double *m) {
             v[c] = a[base | ((c & 1) ? b0 : 0) | ((c & 2) ? b1 : 0) | ((c & 4) ? b2 : 0) | ((c & 8) ? b3 : 0)];
 #pragma unroll
         for (int r = 0; r < D; r++) {
-            if (M::same(r)) continue;
             DGQJ_R re = 0, im = 0;
             bool some = false;
 #pragma unroll

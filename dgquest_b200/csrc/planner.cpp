@@ -751,7 +751,7 @@ bool encodeBlock(const BlockPlan &block, int numBits, int numReal, int tileBits,
                 const auto &m = pool.mats[(size_t) g.multiIndex];
                 coef.insert(coef.end(), m.begin(), m.end());
                 if (folds == Folding::Specialised && !paired) {
-                    op.selLoc = kDenseAnyBits;
+                    op.selLoc = (uint16_t) (kDenseAnyBits | g.multiShape << 8);
                     for (int i = 0; i < g.numMultiTargets; i++)
                         for (int b = 0; b < kRegBits; b++)
                             if (L.regPos[b] == tm.local[g.multiTargets[i]]) op.selLoc |= (uint16_t) (b << (2 * i));

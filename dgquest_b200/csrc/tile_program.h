@@ -46,7 +46,8 @@ enum KOpKind : uint8_t {
     KOP_PH = 9,    // multiply by (c + i s)
     KOP_Z2 = 10,   // multiply by (c - i s) when the selector bit is 0, (c + i s) when 1
     KOP_DENSE = 11, // dense 2^k x 2^k on register bits 0..k-1 (k = op.k), coefficients re/im; with
-                    // selLoc & kDenseAnyBits, matrix bit i on register bit (selLoc >> 2 i) & 3
+                    // selLoc & kDenseAnyBits, matrix bit i on register bit (selLoc >> 2 i) & 3 and only the
+                    // entries of MatrixShape (selLoc >> 8) & 3
     // Uncontrolled gates with their scalar factor moved into the sweep's
     // global factor (TileProgram::globalRe/Im), leaving unit entries:
     KOP_RY1 = 12,  // [[1, -t], [t, 1]]        (Ry with |cos| >= |sin|, t = tan)
