@@ -646,7 +646,16 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
     // requests of 28..33 qubits took 2.8 s on average); at 2^32 and above
     // the interpreted sweeps themselves take seconds
     const int policy = g_specPolicy.load();
-    const bool cachedOnly = specialise && wantJit && policy >= 1 && s.numBits < 32;
+    // With a unitary wider than a register phase in the list, policy 0 does the
+    // same: the layers between dense sweeps are a few tile sweeps, and compiling
+    // them first costs more than everything else in the circuit (first pass of
+    // a layer and four 6-qubit unitaries, 26 qubits complex128 224 -> 9.0 ms, 29
+    // qubits complex64 342 -> 24.7 ms; 37.8 and 363 ms before tiles were chosen
+    // here). The form choice prices them as specialised sweeps, which is what
+    // later plans run: 7.0 and 16.0 ms.
+    const bool behind = policy == 0 && s.stats.formAuto && formK == 0 &&
+                        std::any_of(s.pending.begin(), s.pending.end(), isWide);
+    const bool cachedOnly = specialise && wantJit && (policy >= 1 || behind) && s.numBits < 32;
     // launching while planning: not when the plan may be redone (policy 1
     // falls back to the interpreting kernel when a kernel is missing; the
     // paired form falls back on a multi-qubit unitary on bit 0) nor with dense
@@ -743,7 +752,7 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
                 which.push_back(i);
             }
         if (cachedOnly && !dgq::jitAllReady(sources)) {
-            if (policy == 1) dgq::jitCompileInBackground(sources);
+            if (policy == 1 || behind) dgq::jitCompileInBackground(sources);
             // the interpreting kernel runs unpaired programs of W <= 12, with
             // diagonal gates where it spends least on them
             code = build(false, true);

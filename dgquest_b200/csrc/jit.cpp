@@ -12,6 +12,7 @@
 #include <functional>
 #include <mutex>
 #include <sstream>
+#include <system_error>
 #include <thread>
 #include <unordered_map>
 
@@ -1215,8 +1216,12 @@ void jitCompileInBackground(const std::vector<std::string> &sources) {
     unsigned hw = std::thread::hardware_concurrency();
     const size_t maxWorkers = std::max(1u, std::min(8u, hw / 2));
     while (c.pool.size() < maxWorkers && c.queue.size() > c.pool.size()) {
+        try {
+            c.pool.emplace_back(backgroundWorker);
+        } catch (const std::system_error &) {
+            break;  // no more threads: the workers there are (or none) take the queue
+        }
         c.alive++;
-        c.pool.emplace_back(backgroundWorker);
     }
     c.work.notify_all();
 }

@@ -54,6 +54,51 @@ def test_cached_only_policy(quest, env, single):
         Q.dgq_setSpecialisationMinBits(-1 if prev_bits == 22 else prev_bits)
 
 
+@pytest.mark.parametrize("single", [False, True])
+def test_tiles_around_wide_unitaries_compile_behind(quest, env, single):
+    """Policy 0, a layer of gates and unitaries wider than a register phase,
+    the form left to the predictor: no pass waits for a compile, and later
+    passes run the kernels compiled meanwhile."""
+    Q, n = quest, 15
+    prev_bits = Q.dgq_setSpecialisationMinBits(1)
+    gen = np.random.default_rng(61)
+    ops = C.random_layers(n, 2, C.config_seed(2, 6160 + int(single)))  # a structure no other test plans
+    blocks = [(gen.choice(n, 6, replace=False).tolist(), C.random_unitary(gen, 64)) for _ in range(2)]
+    o = oracle.Oracle(n)
+    o.apply(ops)
+    for targs, u in blocks:
+        o.multi_qubit_unitary(targs, u)
+    ref = o.amps()
+    o.close()
+    try:
+        def run():
+            q = Q.dgq_createQuregF32(n, env) if single else Q.createQureg(n, env)
+            Q.apply_circuit(q, ops)
+            for targs, u in blocks:
+                m = Q.matrixN(u)
+                Q.multiQubitUnitary(q, Q.int_array(targs), 6, m)
+                Q.destroyComplexMatrixN(m)
+            Q.dgq_planPending(q)
+            st = Q.plan_stats(q)
+            Q.dgq_launchPlanned(q)
+            amps = Q.state_vector(q)
+            Q.destroyQureg(q, env)
+            assert st.formK == 0 and st.jitCompiled == 0
+            if single:
+                assert abs(np.vdot(ref, amps)) ** 2 >= 1 - 1e-6 and abs(np.vdot(amps, amps).real - 1) <= 1e-5
+            else:
+                assert np.abs(amps - ref).max() <= 1e-12
+            return st
+
+        assert run().jitReused == 0
+        deadline = time.time() + 120
+        while not run().jitReused and time.time() < deadline:
+            time.sleep(0.5)
+        assert run().jitReused > 0
+    finally:
+        Q.dgq_setSpecialisationMinBits(-1 if prev_bits == 22 else prev_bits)
+
+
 def test_exit_with_background_compiles_in_flight(quest):
     """A process that exits while background compiles are still queued or
     running (specialisation policy 1) ends cleanly: the binding's exit hook
