@@ -269,7 +269,10 @@ void GateDag::refreshFlat() const {
 // 55 % of a plan's time, most of it in mispredicted branches).
 typedef u64 Sets8 __attribute__((vector_size(64)));
 
-__attribute__((target_clones("arch=x86-64-v4", "avx2", "default"))) static void countAllowed8(
+#if defined(__x86_64__)
+__attribute__((target_clones("arch=x86-64-v4", "avx2", "default")))
+#endif
+static void countAllowed8(
     const u64 *touch, const u64 *cost, size_t n, u64 all, const u64 *allowed, size_t *counts) {
     Sets8 outside, blocked = {}, free = {};
     for (int k = 0; k < 8; k++) outside[k] = ~allowed[k];

@@ -1,8 +1,10 @@
 """CPU tests of the C ABI: libdgq.so loads and exports every function that
 include/QuEST.h and include/dgq.h declare (no GPU calls are made)."""
 import ctypes
+import glob
 import os
 import re
+import subprocess
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -41,3 +43,13 @@ def test_python_mirror_binds_every_symbol():
     for name in declared_functions():
         assert hasattr(quest, name), name
     assert lib.getQuEST_PREC() == 2
+
+
+def test_no_x86_only_attribute_on_other_hosts():
+    # as a compiler for another host sees the C++ sources (headers left out)
+    for path in sorted(glob.glob(os.path.join(ROOT, "dgquest_b200", "csrc", "*.cpp"))):
+        with open(path) as f:
+            text = "".join(line for line in f if not line.lstrip().startswith("#include"))
+        out = subprocess.run(["g++", "-E", "-P", "-U__x86_64__", "-x", "c++", "-"], input=text, capture_output=True,
+                             text=True, check=True).stdout
+        assert "target_clones" not in out and "__builtin_ia32" not in out, path
