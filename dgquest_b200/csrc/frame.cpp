@@ -169,9 +169,13 @@ struct Framer {
         over(m + 6, e);
         over(m + 2, pp);
         over(m + 4, l);
-        // U must be unitary to rounding: |e| = 1 and m2 / m0 = -e conj(p)
-        if (std::fabs(e[0] * e[0] + e[1] * e[1] - 1.0) > 1e-14 || std::fabs(l[0] + e[0] * pp[0] + e[1] * pp[1]) > 1e-14 ||
-            std::fabs(l[1] + e[1] * pp[0] - e[0] * pp[1]) > 1e-14)
+        // U must be unitary to rounding: |e| = 1 and m2 / m0 = -e conj(p), whose
+        // residuals are dropped. Of 20000 random unitaries rounded to doubles
+        // none has more than 1.9e-15 (2 % more than 9e-16), of products of two
+        // one in 2000 more than 2e-15; matrices further off run as given.
+        const double tol = 2e-15;
+        if (std::fabs(e[0] * e[0] + e[1] * e[1] - 1.0) > tol || std::fabs(l[0] + e[0] * pp[0] + e[1] * pp[1]) > tol ||
+            std::fabs(l[1] + e[1] * pp[0] - e[0] * pp[1]) > tol)
             return false;
         global(m[0], m[1]);
         pair(FK_RN, q, pp[0], pp[1]);

@@ -117,7 +117,8 @@ struct FrameSweep {
 
 // The framed form of a tile program of width W (unpaired, W <= 12); false
 // when an op has none (dense ops, controlled rotations and general 2x2 ops,
-// controlled Y, X with several controls, 2x2 matrices unitary only to 1e-14).
+// controlled Y, X with several controls, 2x2 matrices that are not unitary to
+// rounding) or there are more than kFrameMaxOps.
 bool frameProgram(const TileProgram &p, int W, FrameSweep &out);
 
 // The sweep on the host, on 2^numBits amplitudes (re, im pairs).

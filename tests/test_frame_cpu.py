@@ -80,3 +80,14 @@ def test_phases_on_many_qubits_are_framed(n, w, seed):
     got, sweeps = ir.frame_apply_host(n, w, *arrays, a)
     assert sweeps >= 1
     assert np.abs(got - want).max() <= 1e-12
+
+
+@pytest.mark.parametrize("entry", [2, 4, 6])
+def test_matrices_off_unitarity_beyond_rounding_run_as_given(entry):
+    # a general 2x2 is framed as a unitary, so one that is not to rounding
+    # (within what the API accepts) has no framed form
+    u = C.random_unitary(np.random.default_rng(3), 2).ravel()
+    p = np.stack([u.real, u.imag], -1).ravel()
+    assert framed(9, 9, C.OpList().add(C.UNITARY, 3, p=p).array())[1] == 1
+    p[entry:entry + 2] *= 1 + 1e-14
+    assert framed(9, 9, C.OpList().add(C.UNITARY, 3, p=p).array())[1] == 0
