@@ -14,8 +14,8 @@
 // The state and the output must live on the device that is current when
 // the call is made (checked with cudaPointerGetAttributes, a host query);
 // the scratch is that device's copy of the array.
-// The array holds kStaticProbCtas x 17 doubles (2,228,224 bytes = 2.125 MiB)
-// and stays resident on every GPU that loads libdgq until the process exits.
+// The array holds kStaticProbCtas x kProbSlots doubles (655,360 bytes = 640
+// KiB) and stays resident on every GPU that loads libdgq until the process exits.
 // That bounds the state to 2^30 amplitudes (numBits <= 30). All calls share
 // the array and it keeps the last call's partial sums; nothing in it needs
 // to start at zero (each CTA writes every slot it owns before the finalise
@@ -32,10 +32,10 @@
 
 namespace dgq {
 
-constexpr int kStaticProbCtas = 1 << 14;     // 2^30 amplitudes at 2^16 per CTA
+constexpr int kStaticProbCtas = 1 << 12;     // 2^30 amplitudes at 2^18 per CTA (probShape)
 constexpr int kStaticProbMaxBits = 30;
 
-static __device__ __align__(256) double g_probScratch[kStaticProbCtas * 17];
+static __device__ __align__(256) double g_probScratch[kStaticProbCtas * kProbSlots];
 
 // host-side copy of the scratch array's device address, per device
 static std::mutex g_scratchMutex;
@@ -54,8 +54,8 @@ extern "C" int dgq_calcProbOfAllZeroNoAlloc(const void *deviceState, int numBits
     }
     if (numBits < 1 || numBits > kStaticProbMaxBits) {
         char msg[160];
-        snprintf(msg, sizeof msg, "numBits = %d is outside 1..%d, the size the static scratch (%d x 17 doubles) holds",
-                 numBits, kStaticProbMaxBits, kStaticProbCtas);
+        snprintf(msg, sizeof msg, "numBits = %d is outside 1..%d, the size the static scratch (%d x %d doubles) holds",
+                 numBits, kStaticProbMaxBits, kStaticProbCtas, kProbSlots);
         raiseExternal(104, __func__, msg);
         return -1;
     }

@@ -197,7 +197,7 @@ int dgq_measureFp64Peak(double *tflops);
  * device that is current at the call (checked; another GPU's memory is
  * rejected). stream: a cudaStream_t (NULL = default stream); results are
  * ready when the stream reaches them. The partial sums go to a static
- * device array of 16384 x 17 doubles (2.125 MiB, resident on every GPU that
+ * device array of 4096 x 20 doubles (640 KiB, resident on every GPU that
  * loads the library until the process exits), so numBits is limited to
  * 1..30; larger states are rejected. The first call on each device looks up
  * that array's device address (make that first call before any stream

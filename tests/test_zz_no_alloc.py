@@ -52,6 +52,23 @@ def test_no_alloc_matches_regular_readout_twice(quest, env):
         quest.destroyQureg(q, env)
 
 
+@pytest.mark.parametrize("n", [23, 30])
+def test_no_alloc_fills_its_scratch(quest, env, n):
+    # the most CTAs with one unit each, and the largest state it takes (16 GiB)
+    import torch
+    if torch.cuda.mem_get_info()[0] < (20 << n):
+        pytest.skip("not enough device memory")
+    b = C.OpList()
+    for t in range(n):
+        b.add(C.RY, t, p=(0.1 + 0.05 * t,))
+    q = quest.createQureg(n, env)
+    C.replay(q, b.array())
+    got, _ = _probs_no_alloc(quest, q, torch)
+    quest.destroyQureg(q, env)
+    assert np.abs(got[:n] - np.cos(0.05 + 0.025 * np.arange(n)) ** 2).max() <= TOL
+    assert abs(got[n] - 1.0) <= TOL
+
+
 def test_no_alloc_rejects_oversized_state(quest, env):
     q = quest.createQureg(10, env)
     nb = ctypes.c_int(0)
