@@ -264,16 +264,18 @@ void GateDag::refreshFlat() const {
     flatValid_ = true;
 }
 
-// One scan for 8 candidate sets, without branches: with 256- or 512-bit
-// vectors a gate costs the eight sets little more than one (the scans were
-// 55 % of a plan's time, most of it in mispredicted branches).
+// Insertion order is a topological order, so one forward pass decides
+// which gates are reachable inside `allowed`: a gate held back holds back
+// every later gate on its qubits. One scan for 8 candidate sets, without
+// branches: with 256- or 512-bit vectors a gate costs the eight sets little
+// more than one (the scans were 55 % of a plan's time, most of it in
+// mispredicted branches).
 typedef u64 Sets8 __attribute__((vector_size(64)));
 
 #if defined(__x86_64__)
 __attribute__((target_clones("arch=x86-64-v4", "avx2", "default")))
 #endif
-static void countAllowed8(
-    const u64 *touch, const u64 *cost, size_t n, u64 all, const u64 *allowed, size_t *counts) {
+static void countAllowed8(const u64 *touch, const u64 *cost, size_t n, u64 all, const u64 *allowed, size_t *counts) {
     Sets8 outside, blocked = {}, free = {};
     for (int k = 0; k < 8; k++) outside[k] = ~allowed[k];
     for (size_t i = 0; i < n;) {
@@ -303,32 +305,6 @@ void GateDag::countAllowed(const u64 *allowed, size_t total, size_t *counts) con
         countAllowed8(flatTouch_.data(), flatCost_.data(), flatTouch_.size(), all, set, count);
         std::copy(count, count + m, counts + c);
     }
-}
-
-// Insertion order is a topological order, so one forward pass decides
-// which gates are reachable inside `allowed`: a gate held back holds back
-// every later gate on its qubits.
-size_t GateDag::countAllowed(u64 allowed) const {
-    refreshFlat();
-    const size_t n = flatTouch_.size();
-    const u64 *touch = flatTouch_.data(), *cost = flatCost_.data();
-    const u64 all = numQubits_ >= 64 ? ~0ULL : ((1ULL << numQubits_) - 1);
-    u64 blocked = 0;
-    size_t count = 0;
-    for (size_t i = 0; i < n && blocked != all; i++) {
-        if ((touch[i] & blocked) || (cost[i] & ~allowed)) {
-            blocked |= touch[i];
-            continue;
-        }
-        count++;
-    }
-    return count;
-}
-
-u64 GateDag::frontierTargets(u64 allowed) const {
-    u64 frontier = 0;
-    for (u64 m : frontierSets(allowed)) frontier |= m;
-    return frontier;
 }
 
 std::vector<u64> GateDag::frontierSets(u64 allowed) const {

@@ -40,13 +40,12 @@ public:
     std::vector<Gate> gatesInOrder() const;
 
     // Gates of the largest dependency-closed set whose non-diagonal targets
-    // all lie in `allowed` (count only / remove and return them).
-    size_t countAllowed(u64 allowed) const;
+    // all lie in `allowed`: their number for each of n sets, in one scan for
+    // every 8, and taking them (remove and return).
+    void countAllowed(const u64 *allowed, size_t n, size_t *counts) const;
     std::vector<Gate> takeAllowed(u64 allowed);
-    // Non-diagonal target bits of the gates that could run next if their
-    // targets were allowed (frontier of the allowed-closed set).
-    u64 frontierTargets(u64 allowed) const;
-    // The distinct sets of missing target bits of those next gates.
+    // The distinct sets of missing target bits of the gates that could run
+    // next if their targets were allowed (frontier of the allowed-closed set).
     std::vector<u64> frontierSets(u64 allowed) const;
     // With touchCost, the queries above count every qubit a gate touches
     // (targets, controls, diagonal gates' qubits) instead of its
@@ -56,9 +55,6 @@ public:
         touchCost_ = on;
         flatValid_ = false;
     }
-
-    // countAllowed for each of n sets, in one scan for every 8.
-    void countAllowed(const u64 *allowed, size_t n, size_t *counts) const;
 
 private:
     // Alive nodes in insertion order as (touched qubits, non-diagonal

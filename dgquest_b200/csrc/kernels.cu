@@ -431,8 +431,9 @@ __global__ void pageSwapKernel(V *__restrict__ a, V *__restrict__ b, int pageBit
 // --------------------------------------------------- bit-pair exchange
 // The amplitude at each index moves to the index with the bits of every pair
 // exchanged, in place. A tile spans the lowest address bits and their
-// partners, so that runs of at least 128 bytes are read and written whole
-// whichever bits trade places; a CTA holds a tile and the one it trades with
+// partners, so that runs of at least 128 bytes (64 in complex64 registers of
+// up to 14 bits, whose tiles are of 2^6) are read and written whole whichever
+// bits trade places; a CTA holds a tile and the one it trades with
 // in shared memory and stores each in the other's place, permuted.
 // Bound: HBM, every amplitude read and written once. (One thread per pair of
 // amplitudes touched 16 bytes of a 64-byte DRAM access at one of the two ends

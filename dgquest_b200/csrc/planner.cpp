@@ -91,10 +91,11 @@ static void growMask(const GateDag &dag, u64 &mask, int budget, bool preferHigh,
 }
 
 // Grows `mask` keeping the `width` masks of each size that let the most gates
-// run, and takes the best of all. Greedy growth commits to every bit: on 30
-// qubits at depth 20 a width of 16 saves 0..2 of 18 sweeps, 4 saves 4 of 17
-// on a 26-qubit ansatz of depth 10, and on a 4 x 7 grid greedy growth is the
-// better one (12 sweeps, 13), so the cost model plans with each.
+// run, and takes the best of all. Greedy growth commits to every bit, but no
+// search is the best throughout, so the cost model plans with each. Sweeps of
+// 12-bit tiles, greedy / with a step of lookahead / widths 4 / 16: 30 qubits at
+// depth 20 19 / 18 / 19 / 17, a 26-qubit ansatz of depth 10 14 / 17 / 13 / 16,
+// grids of depth 16, 4 x 7 14 / 14 / 13 / 13, 5 x 6 14 / 15 / 14 / 15.
 static void beamMask(const GateDag &dag, u64 &mask, int budget, size_t width) {
     std::vector<u64> beam{mask}, sets, next;
     std::vector<size_t> counts, rank;
