@@ -4,7 +4,9 @@ and Pauli gates between rotations on tile, thread and CTA bits, a collapse
 between two parts, and batches that are framed or not, against the oracle.
 
 Bound: the same factors as the gate-by-gate product, so 1e-12 per amplitude
-in complex128 and fidelity 1 - 1e-6 in complex64."""
+in complex128. In complex64 each of G gates rounds its products and sums at
+most 4 times, 2^-24 of the state each: 4 G 2^-24 in the 2-norm of the
+difference, with no normalisation, so a wrong overall factor shows."""
 import numpy as np
 import pytest
 
@@ -17,9 +19,9 @@ FRAMED = [C.H, C.X, C.Y, C.Z, C.S, C.T, C.RX, C.RY, C.RZ, C.PHASE, C.CNOT, C.CNO
           C.SQW, C.COMPACT, C.UNITARY, C.SWAP]
 
 
-def check(amps, ref, single):
+def check(amps, ref, single, gates=0):
     if single:
-        assert abs(np.vdot(ref, amps)) ** 2 / np.vdot(amps, amps).real >= 1 - 1e-6
+        assert gates and np.linalg.norm(amps - ref) <= 4 * gates * 2.0 ** -24
     else:
         assert np.abs(amps - ref).max() <= 1e-12
 
@@ -37,7 +39,7 @@ def test_framed_sweeps_match_oracle(quest, env, n, width, single):
         amps = Q.state_vector(q)
     finally:
         Q.destroyQureg(q, env)
-    check(amps, oracle.run(n, ops)[0], single)
+    check(amps, oracle.run(n, ops)[0], single, len(ops))
 
 
 def test_collapse_between_framed_sweeps(quest, env):
@@ -58,14 +60,15 @@ def test_collapse_between_framed_sweeps(quest, env):
     check(amps, ref[0], False)
 
 
+@pytest.mark.parametrize("single", [False, True])
 @pytest.mark.parametrize("unframed", [False, True])
-def test_batches_with_and_without_a_framed_form(quest, env, unframed):
+def test_batches_with_and_without_a_framed_form(quest, env, unframed, single):
     Q = quest
     sizes = [9, 10, 12, 13, 14]
     lists = [C.mixed_ops(n, 200, 40 + n, kinds=FRAMED) for n in sizes]
     if unframed:
         lists[2] = np.concatenate([lists[2], C.mixed_ops(sizes[2], 5, 9, kinds=[C.CRX])])
-    regs = [Q.createQureg(n, env) for n in sizes]
+    regs = [(Q.dgq_createQuregF32 if single else Q.createQureg)(n, env) for n in sizes]
     try:
         for q, ops in zip(regs, lists):
             C.replay(q, ops)
@@ -78,7 +81,7 @@ def test_batches_with_and_without_a_framed_form(quest, env, unframed):
         for q in regs:
             Q.destroyQureg(q, env)
     for n, ops, a in zip(sizes, lists, states):
-        check(a, oracle.run(n, ops)[0], False)
+        check(a, oracle.run(n, ops)[0], single, len(ops))
 
 
 @pytest.mark.parametrize("unframed", [False, True])
@@ -146,11 +149,12 @@ def test_phases_on_many_qubits(quest, env, n, width, single):
                         Q.multiControlledPhaseShift(q, Q.int_array(qubits), k, angle)
         want = o.amps()
         o.close()
-        check(Q.state_vector(regs[0]), want, single)
+        gates = 5 * (20 + 3)
+        check(Q.state_vector(regs[0]), want, single, gates)
         b = Q.Batch(regs[1:], config={"tileBits": width})
         b.launch()
         b.wait()
-        check(Q.state_vector(regs[1]), want, single)
+        check(Q.state_vector(regs[1]), want, single, gates)
         b.close()
     finally:
         for q in regs:
