@@ -653,7 +653,8 @@ bool planPending(QuregState &s, const char *func, bool specialise, bool launch) 
     // qubits complex64 342 -> 24.7 ms; 37.8 and 363 ms before tiles were chosen
     // here). The form choice prices them as specialised sweeps, which is what
     // later plans run: 7.0 and 16.0 ms.
-    const bool behind = policy == 0 && s.stats.formAuto && formK == 0 &&
+    // (A plan that is kept to be launched again, dgq_planPending, compiles first.)
+    const bool behind = launch && policy == 0 && s.stats.formAuto && formK == 0 &&
                         std::any_of(s.pending.begin(), s.pending.end(), isWide);
     const bool cachedOnly = specialise && wantJit && (policy >= 1 || behind) && s.numBits < 32;
     // launching while planning: not when the plan may be redone (policy 1

@@ -249,7 +249,8 @@ int dgq_frameApplyHost(int numQubits, int tileBits, int count, const int32_t *ty
 int dgq_setSpecialisationMinBits(int minBits);
 /* 0 (default): plans that need specialised kernels compile them before
  * running, except those that the form choice leaves as tiles around unitaries
- * of more than 4 targets, which run as under 1. 1: a plan runs specialised only if its kernels are compiled
+ * of more than 4 targets, which run as under 1 unless they are planned by
+ * dgq_planPending to be launched again. 1: a plan runs specialised only if its kernels are compiled
  * already; otherwise it runs the interpreting kernel while its kernels
  * compile on background host threads for later plans of the same structure
  * (for serving one-off circuits); registers of >= 32 address bits still

@@ -54,15 +54,17 @@ def test_cached_only_policy(quest, env, single):
         Q.dgq_setSpecialisationMinBits(-1 if prev_bits == 22 else prev_bits)
 
 
+@pytest.mark.parametrize("kept", [False, True])
 @pytest.mark.parametrize("single", [False, True])
-def test_tiles_around_wide_unitaries_compile_behind(quest, env, single):
-    """Policy 0, a layer of gates and unitaries wider than a register phase,
-    the form left to the predictor: no pass waits for a compile, and later
-    passes run the kernels compiled meanwhile."""
+def test_tiles_around_wide_unitaries_compile_behind(quest, env, single, kept):
+    """Policy 0, layers of gates and unitaries wider than a register phase, the
+    form left to the predictor: no pass waits for a compile, and later passes
+    run the kernels compiled meanwhile. A plan that is kept to be launched
+    again has its kernels at once."""
     Q, n = quest, 15
     prev_bits = Q.dgq_setSpecialisationMinBits(1)
     gen = np.random.default_rng(61)
-    ops = C.random_layers(n, 2, C.config_seed(2, 6160 + int(single)))  # a structure no other test plans
+    ops = C.random_layers(n, 2, C.config_seed(2, 6160 + int(single) + 2 * int(kept)))  # no other test plans it
     blocks = [(gen.choice(n, 6, replace=False).tolist(), C.random_unitary(gen, 64)) for _ in range(2)]
     o = oracle.Oracle(n)
     o.apply(ops)
@@ -78,23 +80,28 @@ def test_tiles_around_wide_unitaries_compile_behind(quest, env, single):
                 m = Q.matrixN(u)
                 Q.multiQubitUnitary(q, Q.int_array(targs), 6, m)
                 Q.destroyComplexMatrixN(m)
-            Q.dgq_planPending(q)
-            st = Q.plan_stats(q)
-            Q.dgq_launchPlanned(q)
+            if kept:
+                Q.dgq_planPending(q)
+                Q.dgq_launchPlanned(q)
             amps = Q.state_vector(q)
+            st = Q.plan_stats(q)
             Q.destroyQureg(q, env)
-            assert st.formK == 0 and st.jitCompiled == 0
+            assert st.formK == 0
             if single:
                 assert abs(np.vdot(ref, amps)) ** 2 >= 1 - 1e-6 and abs(np.vdot(amps, amps).real - 1) <= 1e-5
             else:
                 assert np.abs(amps - ref).max() <= 1e-12
-            return st
+            return st.jitCompiled, st.jitReused
 
-        assert run().jitReused == 0
-        deadline = time.time() + 120
-        while not run().jitReused and time.time() < deadline:
-            time.sleep(0.5)
-        assert run().jitReused > 0
+        if kept:
+            assert run()[0] > 0 and run()[0] == 0
+        else:
+            assert run() == (0, 0)
+            deadline = time.time() + 120
+            while run() == (0, 0) and time.time() < deadline:
+                time.sleep(0.5)
+            compiled, reused = run()
+            assert compiled == 0 and reused > 0
     finally:
         Q.dgq_setSpecialisationMinBits(-1 if prev_bits == 22 else prev_bits)
 
